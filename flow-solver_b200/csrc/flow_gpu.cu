@@ -197,12 +197,8 @@ struct flow_ctx {
   ChunkTables ct{};          // mode 3 tables and sweep records
   std::vector<int> h_col_ptr, h_chunk_start;
   int chunk_rows = 0, chunk_levels = 0;  // requested limits (0: defaults)
-  // sub-level tables of each ring shape of the chunk sweep (per direction);
-  // ct.sub_start / ct.chunk_sub point at those of the shape in use
-  const int* ring_sub_start[kRingShapes][2] = {};
-  const int* ring_chunk_sub[kRingShapes][2] = {};
-  bool ring_ok[kRingShapes] = {};
-  int ring = 0;  // requested shape: sub-levels of ring_rows(ring) rows
+  bool ring_ok[kRingShapes] = {};  // CTA shapes of the chunk sweep this mesh may take
+  int ring = 0;                    // requested shape (flow_set_sweep_ring)
   bool grad_written = false;  // the caller wrote the gradient (flow_set "grad")
   int sweep_df = 0;  // 1: one-launch (dataflow) mode 3 sweeps (flow_set_sweep_dataflow)
   bool has_edge_w = false;  // the grid view carried LSQ edge weights
@@ -536,6 +532,31 @@ int launch_residuals(flow_ctx* c, const StepArgs& a, int jac) {
   return rc;
 }
 
+// The mode 3 sweep kernels by lanes a row, CTA shape and direction: one
+// colour, a colour's two passes in a row, a whole sweep in one launch.
+using ChunkKernel = void (*)(DevState, ChunkTables, float*, int, int);
+using ChunkDfKernel = void (*)(DevState, ChunkTables, float*, int, long);
+template <int L>
+struct ChunkKernels {
+  static constexpr int w0 = ring_warps(0), w1 = ring_warps(1), w2 = ring_warps(2);
+  static constexpr ChunkKernel one[kRingShapes][2] = {
+      {k_sweep_chunk<0, L, w0>, k_sweep_chunk<1, L, w0>},
+      {k_sweep_chunk<0, L, w1>, k_sweep_chunk<1, L, w1>},
+      {k_sweep_chunk<0, L, w2>, k_sweep_chunk<1, L, w2>}};
+  static constexpr ChunkKernel pair[kRingShapes][2] = {
+      {k_sweep_chunk_pair<0, L, w0>, k_sweep_chunk_pair<1, L, w0>},
+      {k_sweep_chunk_pair<0, L, w1>, k_sweep_chunk_pair<1, L, w1>},
+      {k_sweep_chunk_pair<0, L, w2>, k_sweep_chunk_pair<1, L, w2>}};
+  static constexpr ChunkDfKernel df[2] = {k_sweep_chunk_df<0, L>, k_sweep_chunk_df<1, L>};
+};
+ChunkKernel chunk_kernel(const ChunkTables& ct, int dir, bool pair) {
+  const auto pick = [&](auto K) { return pair ? K.pair[ct.ring][dir] : K.one[ct.ring][dir]; };
+  return ct.lanes_log2 == 2 ? pick(ChunkKernels<4>()) : pick(ChunkKernels<2>());
+}
+ChunkDfKernel chunk_df_kernel(const ChunkTables& ct, int dir) {
+  return ct.lanes_log2 == 2 ? ChunkKernels<4>::df[dir] : ChunkKernels<2>::df[dir];
+}
+
 // linear_solve (linear_algebra.C:122-401): subits sweeps, alternating
 // forward/backward, each followed by the b-Ax RMS that may stop the loop.
 // Precision form: p->subits multicolour FP32 sweeps from dQ = 0, colours
@@ -547,7 +568,8 @@ int launch_linear_solve_mixed(flow_ctx* c, const flow_params* p) {
   if (c->precision == 3) {
     // coloured chunks of the reference order, in-place FP32 iterate
     const ChunkTables& ct = c->ct;
-    const size_t smem = 16 * kRecStride * kRingRecords + sizeof(float4) * ct.maxwin;
+    const size_t smem = sizeof(float4) * (ct.maxwin + 1);  // a zero, then the window
+    const int threads = 32 * ring_warps(ct.ring);
     if (c->sweep_pairs && !(c->sweep_df && ct.ring == 0) && p->subits > 1) {
       // the (sweep, colour) passes in order; where one sweep ends with the
       // colour the next begins with, the two passes are one launch
@@ -563,21 +585,8 @@ int launch_linear_solve_mixed(flow_ctx* c, const flow_params* p) {
         const int last = (pair ? passes[k + 1].first : it) == p->subits - 1;
         if (pair) k++;
         if (nb <= 0) continue;
-        if (pair) {
-          auto kern = dir == 0 ? (ct.ring == 2 ? k_sweep_chunk_pair<0, 16>
-                                  : ct.ring == 1 ? k_sweep_chunk_pair<0, 32>
-                                                 : k_sweep_chunk_pair<0, 64>)
-                               : (ct.ring == 2 ? k_sweep_chunk_pair<1, 16>
-                                  : ct.ring == 1 ? k_sweep_chunk_pair<1, 32>
-                                                 : k_sweep_chunk_pair<1, 64>);
-          kern<<<nb, 256, smem, c->stream>>>(c->s, ct, c->mt.dq32, col, last);
-        } else {
-          auto kern = dir == 0 ? (ct.ring == 2 ? k_sweep_chunk<0, 16>
-                                  : ct.ring == 1 ? k_sweep_chunk<0, 32> : k_sweep_chunk<0, 64>)
-                               : (ct.ring == 2 ? k_sweep_chunk<1, 16>
-                                  : ct.ring == 1 ? k_sweep_chunk<1, 32> : k_sweep_chunk<1, 64>);
-          kern<<<nb, 256, smem, c->stream>>>(c->s, ct, c->mt.dq32, col, last);
-        }
+        chunk_kernel(ct, dir, pair)<<<nb, threads, smem, c->stream>>>(c->s, ct, c->mt.dq32, col,
+                                                                     last);
         rc |= launch_check(c);
       }
       return rc;
@@ -588,12 +597,8 @@ int launch_linear_solve_mixed(flow_ctx* c, const flow_params* p) {
       if (c->sweep_df && ct.ring == 0) {
         // the whole sweep in one launch, one CTA per chunk
         const long max_spin = 1L << 22;
-        if (dir == 0)
-          k_sweep_chunk_df<0><<<ct.nchunks, 256, smem, c->stream>>>(c->s, ct, c->mt.dq32, last,
-                                                                   max_spin);
-        else
-          k_sweep_chunk_df<1><<<ct.nchunks, 256, smem, c->stream>>>(c->s, ct, c->mt.dq32, last,
-                                                                   max_spin);
+        chunk_df_kernel(ct, dir)<<<ct.nchunks, threads, smem, c->stream>>>(c->s, ct, c->mt.dq32,
+                                                                          last, max_spin);
         rc |= launch_check(c);
         continue;
       }
@@ -601,11 +606,8 @@ int launch_linear_solve_mixed(flow_ctx* c, const flow_params* p) {
         const int col = dir == 0 ? ci : ct.ncol - 1 - ci;
         const int nb = c->h_col_ptr[col + 1] - c->h_col_ptr[col];
         if (nb <= 0) continue;
-        auto kern = dir == 0 ? (ct.ring == 2 ? k_sweep_chunk<0, 16>
-                                : ct.ring == 1 ? k_sweep_chunk<0, 32> : k_sweep_chunk<0, 64>)
-                             : (ct.ring == 2 ? k_sweep_chunk<1, 16>
-                                : ct.ring == 1 ? k_sweep_chunk<1, 32> : k_sweep_chunk<1, 64>);
-        kern<<<nb, 256, smem, c->stream>>>(c->s, ct, c->mt.dq32, col, last);
+        chunk_kernel(ct, dir, false)<<<nb, threads, smem, c->stream>>>(c->s, ct, c->mt.dq32, col,
+                                                                      last);
         rc |= launch_check(c);
       }
     }
@@ -1012,7 +1014,7 @@ bool preload_kernels() {
         (const void*)k_sweep_ordered<false>, (const void*)k_sweep_color32<true>,
         (const void*)k_sweep_color32<false>, (const void*)k_sweep_ordered32<true>,
         (const void*)k_sweep_ordered32<false>, (const void*)k_prepare_sweep32,
-        (const void*)k_fill_sweep_records, (const void*)k_prepare_sweep,
+        (const void*)k_fill_sweep_slots, (const void*)k_prepare_sweep,
         (const void*)k_lin_residual, (const void*)k_finalize_rms, (const void*)k_exact_rms,
         (const void*)k_finish_step,
         (const void*)k_body_forces,
@@ -1029,18 +1031,22 @@ bool ensure_kernel_attrs(int device) {
   if ((int)done.size() <= device) done.resize(device + 1, 0);
   if (done[device]) return true;
   DeviceWide gate(g_device_gate);
-  const int chunk_cap = 227 * 1024 - kChunkStaticSmem;
+  const int chunk_cap = (kChunkWinMax + 1) * (int)sizeof(float4);
   const int cta = (int)sizeof(SweepSmem);
   bool ok = preload_kernels();
-  for (const void* f : {(const void*)k_sweep_chunk_pair<0, 64>, (const void*)k_sweep_chunk_pair<1, 64>,
-                        (const void*)k_sweep_chunk_pair<0, 32>, (const void*)k_sweep_chunk_pair<1, 32>,
-                        (const void*)k_sweep_chunk_pair<0, 16>, (const void*)k_sweep_chunk_pair<1, 16>,
-                        (const void*)k_sweep_chunk_df<0>, (const void*)k_sweep_chunk_df<1>,
-                        (const void*)k_sweep_chunk<0, 64>, (const void*)k_sweep_chunk<1, 64>,
-                        (const void*)k_sweep_chunk<0, 32>, (const void*)k_sweep_chunk<1, 32>,
-                        (const void*)k_sweep_chunk<0, 16>, (const void*)k_sweep_chunk<1, 16>})
-    ok = ok && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    chunk_cap) == cudaSuccess;
+  auto set_chunk_cap = [&](auto K) {
+    std::vector<const void*> fs = {(const void*)K.df[0], (const void*)K.df[1]};
+    for (int shape = 0; shape < kRingShapes; shape++)
+      for (int dir = 0; dir < 2; dir++) {
+        fs.push_back((const void*)K.one[shape][dir]);
+        fs.push_back((const void*)K.pair[shape][dir]);
+      }
+    for (const void* f : fs)
+      ok = ok && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      chunk_cap) == cudaSuccess;
+  };
+  set_chunk_cap(ChunkKernels<4>());
+  set_chunk_cap(ChunkKernels<2>());
   for (const void* f : {(const void*)k_node_stage<1>, (const void*)k_node_stage<3>})
     ok = ok && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)kStageSmemMax) == cudaSuccess;
@@ -1103,7 +1109,7 @@ int build_chunk_tables(flow_ctx* c) {
                                : std::min(2048, std::max(64, ((2 * bw + 63) / 64) * 64));
   const int lmax = c->chunk_levels > 0 ? c->chunk_levels : 32;
   // an automatic chunk size shrinks (64 rows at a time) until every chunk's
-  // window of the iterate fits in shared memory beside the record ring
+  // window of the iterate is within kChunkWinMax
   for (;;) {
     const int rc = build_chunks_with(c, bw, cmax, lmax);
     if (rc != FLOW_ERR_ARG || c->chunk_rows > 0 || cmax - 64 < std::max(64, bw / 2)) return rc;
@@ -1111,16 +1117,9 @@ int build_chunk_tables(flow_ctx* c) {
   }
 }
 
-// Point the chunk tables at the sub-levels of the requested ring shape (the
-// largest shape when the requested one does not fit a chunk).
-void apply_ring(flow_ctx* c) {
-  const int shape = c->ring_ok[c->ring] ? c->ring : 0;
-  for (int dir = 0; dir < 2; dir++) {
-    c->ct.sub_start[dir] = c->ring_sub_start[shape][dir];
-    c->ct.chunk_sub[dir] = c->ring_chunk_sub[shape][dir];
-  }
-  c->ct.ring = shape;
-}
+// The requested CTA shape of the chunk sweep (the largest one when the mesh
+// may not take the requested one).
+void apply_ring(flow_ctx* c) { c->ct.ring = c->ring_ok[c->ring] ? c->ring : 0; }
 
 int build_chunks_with(flow_ctx* c, int bw, int cmax, int lmax) {
   for (int shape = 0; shape < kRingShapes; shape++) c->ring_ok[shape] = true;
@@ -1181,8 +1180,7 @@ int build_chunks_with(flow_ctx* c, int bw, int cmax, int lmax) {
     win[q] = make_int2(a, b);
     maxwin = std::max(maxwin, b - a + 1);
   }
-  const size_t smem = 16 * kRecStride * kRingRecords + sizeof(float4) * maxwin;
-  if (smem + kChunkStaticSmem > 227 * 1024) {
+  if (maxwin > kChunkWinMax) {
     set_error("precision mode 3: a chunk's window does not fit in shared memory (bandwidth too large)");
     return FLOW_ERR_ARG;
   }
@@ -1220,81 +1218,98 @@ int build_chunks_with(flow_ctx* c, int bw, int cmax, int lmax) {
       return FLOW_ERR_CUDA;
     }
   }
-  // per direction: levels, sub-levels, records (static part)
-  std::vector<int> levd(nn + 1);
-  for (int dir = 0; dir < 2; dir++) {
-    std::vector<int> pos(nn + 1, 0), order, lev_start, chunk_lev(nch + 1, 0);
-    order.reserve(nn);
+  // levels and tiles; lev holds each row's level
+  {
+    std::vector<int> order, slot(nn + 1, 0), lev_tile, chunk_lev(nch + 1, 0), levb;
+    std::vector<int2> tile_info;
+    // lanes a row by the mean width of a level (k_sweep_chunk)
+    long nlevels = 0;
+    for (int q = 0; q < nch; q++) {
+      int l = 0;
+      for (int j = start[q]; j < start[q + 1]; j++) l = std::max(l, lev[j] + 1);
+      nlevels += l;
+    }
+    const int lanes = nn >= kWideLevel * nlevels ? 2 : 4;
+    const int trows = tile_rows(lanes);
+    ct.lanes_log2 = lanes == 4 ? 2 : 1;
+    order.reserve(nn + nn / 4);
+    std::vector<std::vector<int>> rows_of;
     for (int q = 0; q < nch; q++) {
       const int lo = start[q], hi = start[q + 1] - 1;
       int nlev = 0;
-      for (int t = 0; t <= hi - lo; t++) {
-        const int j = dir == 0 ? lo + t : hi - t;
-        int l = 0;
-        for (int k = ia[j]; k < ia[j + 1]; k++) {
-          const int o = ja[k];
-          const bool up = dir == 0 ? (o >= lo && o < j) : (o <= hi && o > j);
-          if (up) l = std::max(l, levd[o] + 1);
-        }
-        levd[j] = l;
-        nlev = std::max(nlev, l + 1);
-      }
+      for (int j = lo; j <= hi; j++) nlev = std::max(nlev, lev[j] + 1);
+      if ((int)rows_of.size() < nlev) rows_of.resize(nlev);
+      for (int l = 0; l < nlev; l++) rows_of[l].clear();
+      for (int j = lo; j <= hi; j++) rows_of[lev[j]].push_back(j);
       for (int l = 0; l < nlev; l++) {
-        lev_start.push_back((int)order.size());
-        for (int j = lo; j <= hi; j++) {
-          if (levd[j] != l) continue;
-          pos[j] = (int)order.size();
+        lev_tile.push_back((int)order.size() / trows);
+        for (int j : rows_of[l]) {
+          slot[j] = (int)order.size();
           order.push_back(j);
         }
+        while (order.size() % trows) order.push_back(0);
+        tile_info.resize(order.size() / trows, make_int2(q, l));
       }
-      chunk_lev[q + 1] = (int)lev_start.size();
-    }
-    lev_start.push_back((int)order.size());
-    // sub-levels of each ring shape: every level cut into runs of at most
-    // ring_rows(shape) rows (rows of one level are independent, so the cut
-    // changes the barriers, not the arithmetic)
-    for (int shape = 0; shape < kRingShapes; shape++) {
-      const int rows = ring_rows(shape);
-      std::vector<int> ss, cs(nch + 1, 0);
-      bool fits = true;
-      for (int q = 0; q < nch; q++) {
-        cs[q] = (int)ss.size();
-        for (int L = chunk_lev[q]; L < chunk_lev[q + 1]; L++)
-          for (int x = lev_start[L]; x < lev_start[L + 1]; x += rows) ss.push_back(x);
-        if ((int)ss.size() - cs[q] > kChunkSubMax) fits = false;
-      }
-      cs[nch] = (int)ss.size();
-      ss.push_back((int)order.size());
-      if (!fits) {
-        if (shape == 0) {
-          set_error("precision mode 3: a chunk has more sub-levels than the sweep kernel holds");
-          return FLOW_ERR_ARG;
+      chunk_lev[q + 1] = (int)lev_tile.size();
+      // A shape is refused when a chunk's levels, cut into runs of its rows,
+      // make more than kChunkSubMax runs in either direction (runs <= levels
+      // + rows / ring_rows, so only long chains need the count).
+      if (nlev + (hi - lo + 1) / ring_rows(kRingShapes - 1) > kChunkSubMax) {
+        levb.assign(hi - lo + 1, 0);
+        std::vector<int> count[2];
+        for (int dir = 0; dir < 2; dir++) {
+          count[dir].assign(nlev, 0);
+          for (int t = 0; t <= hi - lo; t++) {
+            const int j = dir == 0 ? lo + t : hi - t;
+            int l = lev[j];
+            if (dir == 1) {
+              l = 0;
+              for (int k = ia[j]; k < ia[j + 1]; k++)
+                if (ja[k] > j && ja[k] <= hi) l = std::max(l, levb[ja[k] - lo] + 1);
+              levb[j - lo] = l;
+            }
+            count[dir][l]++;
+          }
+          for (int shape = 0; shape < kRingShapes; shape++) {
+            int runs = 0;
+            for (int n : count[dir]) runs += (n + ring_rows(shape) - 1) / ring_rows(shape);
+            if (runs <= kChunkSubMax) continue;
+            if (shape == 0) {
+              set_error("precision mode 3: a chunk has more sub-levels than the sweep kernel holds");
+              return FLOW_ERR_ARG;
+            }
+            c->ring_ok[shape] = false;
+          }
         }
-        c->ring_ok[shape] = false;
-        continue;
-      }
-      c->ring_sub_start[shape][dir] = upload_vec(c, ss);
-      c->ring_chunk_sub[shape][dir] = upload_vec(c, cs);
-      if (!c->ring_sub_start[shape][dir] || !c->ring_chunk_sub[shape][dir]) {
-        set_error("precision mode 3: table allocation or upload failed");
-        return carve_error(c);
       }
     }
-    // the records' static part is written on the device from the resident
-    // block pattern: only the order (4 bytes a row) crosses from the host
-    SweepRec* rec = c->buf.alloc<SweepRec>(nn);
+    lev_tile.push_back((int)order.size() / trows);
+    // the slots' columns and row numbers are written on the device from the
+    // resident block pattern: only the order (4 bytes a slot) crosses from
+    // the host
+    const size_t nslots = order.size();
+    const size_t words = nslots / trows * tile_words(lanes);
+    ct.tiles = c->buf.alloc<float4>(words);
+    uint4* cols = c->buf.alloc<uint4>(nslots);
+    unsigned* rows = c->buf.alloc<unsigned>(nslots);
     const int* d_order = upload_vec(c, order);
-    if (rec && d_order) {
-      const long words = (long)nn * kRecInts;
-      k_fill_sweep_records<<<(unsigned)((words + 255) / 256), 256, 0, c->stream>>>(
-          rec, d_order, nn, c->m.ia, c->m.ja);
-      if (cudaGetLastError() != cudaSuccess) rec = nullptr;
-    }
-    ct.rec[dir] = rec;
-    ct.pos[dir] = upload_vec(c, pos);
-    if (!ct.rec[dir] || !ct.pos[dir]) {
+    const int2* d_tile_info = upload_vec(c, tile_info);
+    ct.lev_tile = upload_vec(c, lev_tile);
+    ct.chunk_lev = upload_vec(c, chunk_lev);
+    ct.slot = upload_vec(c, slot);
+    if (!ct.tiles || !cols || !rows || !d_order || !d_tile_info || !ct.lev_tile ||
+        !ct.chunk_lev || !ct.slot || !ct.window) {
       set_error("precision mode 3: table allocation or upload failed");
       return carve_error(c);
+    }
+    ct.cols = cols;
+    ct.rows = rows;
+    k_fill_sweep_slots<<<grid_blocks((int)nslots, 256), 256, 0, c->stream>>>(
+        cols, rows, d_order, (int)nslots, trows, d_tile_info, ct.window, c->m.ia, c->m.ja);
+    if (cudaGetLastError() != cudaSuccess ||
+        cudaMemsetAsync(ct.tiles, 0, sizeof(float4) * words, c->stream) != cudaSuccess) {
+      set_error("precision mode 3: filling the sweep tiles failed");
+      return FLOW_ERR_CUDA;
     }
   }
   if (!ct.col_ptr || !ct.col_chunks || !ct.window) {

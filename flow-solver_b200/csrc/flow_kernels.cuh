@@ -814,7 +814,7 @@ __device__ __forceinline__ void face_flux_approx(double4 g, double gamma, const 
 // q of R; each lane sums its row in the reference's face order.  MIXED (the
 // precision form) writes FP32 off-diagonal blocks and FP32 LU factors with
 // reciprocal pivots instead of the FP64 row: into the mode 1/2 tables
-// (MIXED 1) or into the row's forward and backward sweep records (MIXED 2).
+// (MIXED 1) or into the row's slot of its sweep tile (MIXED 2).
 
 // Row q of face `sub`'s Jacobian block J (JL or JR): FP64, or FP32 entries
 // (JF) widened exactly.
@@ -866,13 +866,13 @@ __device__ __forceinline__ void assemble_row(const DevMesh& m, const DevState& s
   // diagonal block is the row's last, so block k is off-diagonal k - k0)
   const int mpos = MIXED == 1 ? mt.pos[n] : 0;
   const int moff = MIXED == 1 ? mt.offd_ptr[mpos] : 0;
-  SweepRec* rf = MIXED == 2 ? ct.rec[0] + ct.pos[0][n] : nullptr;
-  SweepRec* rb = MIXED == 2 ? ct.rec[1] + ct.pos[1][n] : nullptr;
-  if (MIXED == 2) {
-    const float rh = __double2float_rn(-(r));
-    reinterpret_cast<float*>(&rf->rhs)[q] = rh;
-    reinterpret_cast<float*>(&rb->rhs)[q] = rh;
-  }
+  // mode 3: the row's slot in its sweep tile (the layout of flow_state.h)
+  const int ll = MIXED == 2 ? ct.lanes_log2 : 0, trows = 32 >> ll;
+  const int tslot = MIXED == 2 ? ct.slot[n] : 0, tw = tslot & (trows - 1);
+  float4* tile = MIXED == 2 ? ct.tiles + (long)(tslot >> (5 - ll)) * (37 * trows) : nullptr;
+  const int per = 4 >> ll;  // block rows a lane of the sweep holds
+  float4* tblk = tile + 32 * (q & (per - 1)) + (tw << ll) + (q >> (2 - ll));
+  if (MIXED == 2) reinterpret_cast<float*>(tile + 36 * trows + tw)[q] = __double2float_rn(-(r));
   for (int k = k0; k < k1; k++) {
     double4* out = reinterpret_cast<double4*>(s.LHS + 16 * (long)k) + q;
     if (m.ja[k] == n) {
@@ -886,8 +886,7 @@ __device__ __forceinline__ void assemble_row(const DevMesh& m, const DevState& s
     if (MIXED == 1) {
       reinterpret_cast<float4*>(mt.lhs32 + 16 * (long)(moff + (k - k0)))[q] = b32;
     } else if (MIXED == 2) {
-      rf->a[4 * (k - k0) + q] = b32;
-      rb->a[4 * (k - k0) + q] = b32;
+      tblk[32 * per * (k - k0)] = b32;
     } else {
       *out = make_double4(B0, B1, B2, B3);
     }
@@ -922,8 +921,7 @@ __device__ __forceinline__ void assemble_row(const DevMesh& m, const DevState& s
     if (MIXED == 1) {
       reinterpret_cast<float4*>(mt.lu32 + 16 * (long)mpos)[q] = lu;
     } else {
-      rf->lu[q] = lu;
-      rb->lu[q] = lu;
+      tile[32 * trows + trows * q + tw] = lu;
     }
   } else {
     reinterpret_cast<double4*>(s.LUd + 16 * (long)n)[q] = make_double4(o0, o1, o2, o3);
@@ -1681,180 +1679,304 @@ __global__ void k_prepare_sweep32(DevState s, const float* cur, float* next, int
 }
 
 // Precision form, chunked order (mode 3): one colour of chunks, a CTA per
-// chunk, 64 rows (one per quad of 4 lanes, lane r owning block row r) per
-// pass.  The CTA first copies its window of the FP32 iterate (every row its
-// chunk touches) into shared memory, then walks the chunk's sub-levels in
-// order: the records of sub-level u+S-1 are copied into an S-slot ring with
-// cp.async while sub-level u is computed, so the dependency chain only ever
-// reads shared memory.  The ring holds kRingRecords records in one of three
-// shapes (ROWS rows a sub-level x S slots: 64 x 3, 32 x 6, 16 x 12): smaller
-// sub-levels prefetch further ahead for the same shared memory, at the
-// price of more barriers on levels wider than ROWS rows.  Rows of one sub-level are independent; a barrier
-// separates sub-levels.  Rows of other chunks in the window are not written
-// by any CTA of this launch (chunks of one colour share no block).  Per row
-// the arithmetic is that of k_sweep_color32.
-constexpr int kRecRows = 64;        // rows of a sub-level in the largest ring shape
-constexpr int kRingRecords = 192;   // records the ring holds, whatever its shape
-constexpr int kRingShapes = 3;      // sub-levels of 64, 32 or 16 rows
+// chunk.  The CTA copies its window of the FP32 iterate (every row its chunk
+// touches) into shared memory; its warps take the chunk's tiles round robin
+// in level order, LANES lanes a row, each owning 4 / LANES of a block's rows.
+// Rows of other chunks in the window are not written by any CTA of this launch
+// (chunks of one colour share no block).  Per row the arithmetic is that of
+// k_sweep_color32.
+//
+// A chunk is a chain of up to 32 levels, so what bounds the kernel is the
+// time of one level: window reads, eight block products, the ordered
+// subtraction, the 4x4 solve and the hand-over to the next level (about 380
+// cycles for a level of one tile, of which 150 are the reads and products,
+// 125 the subtraction and solve, 110 the hand-over); on wide levels it is the
+// SM's load/store pipe, which every tile and window word passes once.
+// Everything else is kept off that chain:
+// * a level is handed over by an mbarrier that counts its tiles, so a warp
+//   announces its results before it does anything else, and warps without a
+//   tile in a level take no part in it (a barrier of the CTA would put each
+//   warp's loads between its results and the next level);
+// * behind that a warp loads its next tile's blocks and factors straight into
+//   registers (coalesced, no pass through shared memory), a whole round of
+//   the CTA's warps ahead of their use, and the columns and levels of the
+//   tile after that;
+// * the 4x4 solve of the tile's row w runs in lane w alone: one exchange of
+//   the four sums before it, none after; no select or branch stands between
+//   a row's operands and its result (unused blocks are zeros).
+// Both directions read the same tiles, so a row's values are written and
+// cached once.  Per sweep (4 a step, CUDA events, B200) against one barrier a
+// 64-row run of a level, a copy of the records for each direction and a ring
+// of them in shared memory: 2,116 nodes 49 -> 16 us, 25,760 nodes 67 -> 22 us,
+// 181k nodes 109 -> 34 us, 496k nodes 123 -> 54 us.  Asking L2 for the tiles
+// further ahead measured no gain.
+//
+// LANES: two lanes a row halve the window reads a tile's rows need from the
+// load/store pipe, four shorten the chain.  Two are taken where the levels
+// are wide (kWideLevel rows on average): 181k nodes (53 rows a level) 34 us
+// against 42 with four, 496k (74) 54 against 58, 25,760 (25) 22 both, 2,116
+// (10) 17 against 16.  One lane a row measured 37, 58, 24 and 19 us.
+//
+// The CTA shape (autotuned, ring_warps): 16, 8 or 4 warps.  More warps hold
+// more tiles in flight (wide levels), fewer leave room for other chunks on
+// the SM (narrow levels): 34, 43 and 61 us on 181k nodes, 16 and 16 us with
+// 16 and 8 on 2,116.
+constexpr int kWideLevel = 32;
+constexpr int kRingShapes = 3;
+// rows flow_set_sweep_ring names a shape by, and its warps
 __host__ __device__ constexpr int ring_rows(int shape) { return 64 >> shape; }
-constexpr int kRecInts = (int)(sizeof(SweepRec) / 16);  // 16-byte words per record
-// records sit 704 bytes apart in shared memory (640 + 64 of padding), so the
-// two quads of a half-warp read disjoint bank ranges
-constexpr int kRecStride = kRecInts + 4;
-constexpr int kChunkSubMax = 256;   // sub-levels per chunk (host-checked)
-// shared memory the chunk sweep declares statically (room left for the rest)
-constexpr int kChunkStaticSmem = 2048;
+__host__ __device__ constexpr int ring_warps(int shape) { return 16 >> shape; }
+constexpr int kChunkSubMax = 256;  // levels per chunk the kernel holds (host-checked)
+// The widest window of a chunk (rows).  The chunk boundaries, and so the
+// sweep's order and the iterates, depend on it: it is part of what mode 3
+// computes, not of how.
+constexpr int kChunkWinMax = 5952;
 
-
-// Static part of mode 3's sweep records: record i holds row order[i]'s
-// header (row, off-diagonal block count; the diagonal block is the row's
-// last) and its off-diagonal column indices, every other word zero until
-// assembly writes the values.  One thread per 16-byte word: word 0 the
-// header, 1 the right-hand side, 2-5 the LU factors, 6-7 the columns, 8-39
-// the blocks.
-static_assert(offsetof(SweepRec, cols) == 6 * 16 && offsetof(SweepRec, a) == 8 * 16 &&
-                  sizeof(SweepRec) == 40 * 16,
-              "k_fill_sweep_records assumes the SweepRec word layout");
-__global__ void k_fill_sweep_records(SweepRec* __restrict__ rec, const int* __restrict__ order,
-                                     int nrec, const int* __restrict__ ia,
-                                     const int* __restrict__ ja) {
-  const long w = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (w >= (long)nrec * kRecInts) return;
-  const int i = (int)(w / kRecInts), k = (int)(w - (long)i * kRecInts);
-  int4 v = make_int4(0, 0, 0, 0);
-  if (k == 0 || k == 6 || k == 7) {
-    const int j = order[i];
-    const int k0 = ia[j], nb = ia[j + 1] - k0 - 1;
-    if (k == 0) {
-      v = make_int4(j, nb, 0, 0);
-    } else {
-      const int t0 = 4 * (k - 6);
-      v.x = t0 + 0 < nb ? ja[k0 + t0 + 0] : 0;
-      v.y = t0 + 1 < nb ? ja[k0 + t0 + 1] : 0;
-      v.z = t0 + 2 < nb ? ja[k0 + t0 + 2] : 0;
-      v.w = t0 + 3 < nb ? ja[k0 + t0 + 3] : 0;
-    }
-  }
-  reinterpret_cast<int4*>(rec)[w] = v;
+// A slot's row as its position in the chunk's window (from 1; position 0 holds
+// zeros, which the unused blocks of a row read), its off-diagonal block count 
+// and its level, in one word; the top bit is off in an empty slot.
+__host__ __device__ constexpr unsigned slot_info(int pos, int nb, int level) {
+  return 1u << 31 | (unsigned)level << 20 | (unsigned)nb << 16 | (unsigned)pos;
 }
+__device__ __forceinline__ int slot_pos(unsigned h) { return h & 0xffff; }
+__device__ __forceinline__ int slot_blocks(unsigned h) { return h >> 16 & 15; }
+__device__ __forceinline__ int slot_level(unsigned h) { return h >> 20 & 0x7ff; }
 
-// One chunk q of a mode 3 sweep, run by the whole CTA (256 threads).  The
-// colour-synchronous kernel (DF false) queues the chunk's window of the
-// iterate first and its first sub-levels' records after it; the dataflow
-// kernel (DF true) queues the records first, calls wait_deps() (which
-// returns once the chunk's earlier-colour neighbours have finished this
-// sweep, every thread past a barrier) and only then reads the window.
-// reuse_window: the chunk's window is already in shared memory, current (the
-// CTA's previous pass over the same chunk left it there).
-template <int DIR, int ROWS, bool DF, class Wait>
-__device__ __forceinline__ void sweep_chunk_body(const DevState& s, const ChunkTables& ct,
-                                                 float* dq32, int q, int last, int* ss,
-                                                 Wait&& wait_deps, bool reuse_window = false) {
-  constexpr int SLOTS = kRingRecords / ROWS;
-  static_assert(SLOTS * ROWS == kRingRecords && SLOTS >= 3 && 4 * ROWS <= 256,
-                "ring shape");
-  extern __shared__ __align__(16) unsigned char sweep_smem[];
-  int4* slots = reinterpret_cast<int4*>(sweep_smem);
-  float4* win = reinterpret_cast<float4*>(sweep_smem + 16 * kRecStride * kRingRecords);
-  const int tid = threadIdx.x;
-  const int2 w = ct.window[q];
-  const int nwin = w.y - w.x + 1;
-  float4* X = reinterpret_cast<float4*>(dq32);
-  auto load_window = [&]() {
-    if (!reuse_window)
-      for (int i = tid; i < nwin; i += blockDim.x) cp_async16(win + i, X + w.x + i);
-    cp_async_commit();
-  };
-  if (!DF) load_window();
-  const int S0 = ct.chunk_sub[DIR][q], nsub = ct.chunk_sub[DIR][q + 1] - S0;
-  // the chunk's sub-level starts, read once into shared memory ss (the
-  // caller's kChunkSubMax + 1 ints; they sit on the loop's critical path); a
-  // chunk has at most kChunkSubMax sub-levels
-  for (int i = tid; i <= nsub && i <= kChunkSubMax; i += blockDim.x)
-    ss[i] = ct.sub_start[DIR][S0 + i];
-  __syncthreads();
-  const int4* recs = reinterpret_cast<const int4*>(ct.rec[DIR]);
-  auto issue = [&](int u) {
-    if (u < nsub) {
-      const int r0 = ss[u], words = (ss[u + 1] - r0) * kRecInts;
-      const int4* src = recs + (long)r0 * kRecInts;
-      int4* dst = slots + (u % SLOTS) * ROWS * kRecStride;
-      for (int i = tid; i < words; i += blockDim.x) {
-        const int rr = i / kRecInts, ww = i - rr * kRecInts;
-        cp_async16(dst + rr * kRecStride + ww, src + i);
-      }
-    }
-    cp_async_commit();  // one group per sub-level, empty past the end
-  };
-  for (int k = 0; k < SLOTS - 1; k++) issue(k);
-  const int quad = tid >> 2, r = tid & 3;
-  const int qbase = tid & 31 & ~3;
-  const unsigned qmask = 0xFu << qbase;
-  if (DF) {
-    wait_deps();
-    load_window();
-    cp_async_wait<0>();  // the window and the first sub-levels have landed
-  } else {
-    cp_async_wait<SLOTS - 2>();  // the window and sub-level 0 have landed
-  }
-  __syncthreads();
-  for (int u = 0; u < nsub; u++) {
-    issue(u + SLOTS - 1);  // into the slot sub-level u-1 left
-    if (quad < ss[u + 1] - ss[u]) {
-      const SweepRec& R = *reinterpret_cast<const SweepRec*>(
-          slots + ((u % SLOTS) * ROWS + quad) * kRecStride);
-      const int j = R.hdr.x, nb = R.hdr.y;
-      const int* cols = reinterpret_cast<const int*>(R.cols);
-      float acc = reinterpret_cast<const float*>(&R.rhs)[r];
+// The static part of the tiles: per slot i, the window positions of row
+// order[i]'s off-diagonal columns (the diagonal block is the row's last) and
+// its slot_info; order[i] == 0 is an empty slot (of its tile's level).
+// tile_info: each tile's chunk and level.
+__global__ void k_fill_sweep_slots(uint4* __restrict__ cols, unsigned* __restrict__ rows,
+                                   const int* __restrict__ order, int nslots, int rows_a_tile,
+                                   const int2* __restrict__ tile_info,
+                                   const int2* __restrict__ window, const int* __restrict__ ia,
+                                   const int* __restrict__ ja) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nslots) return;
+  const int j = order[i];
+  const int2 info = tile_info[i / rows_a_tile];
+  unsigned c[kRecBlocks] = {};
+  unsigned h = slot_info(0, 0, info.y) & ~(1u << 31);
+  if (j > 0) {
+    const int w0 = window[info.x].x - 1;  // the row of window position 0
+    const int k0 = ia[j];
+    const int nb = ia[j + 1] - k0 - 1;
 #pragma unroll
-      for (int t = 0; t < kRecBlocks; t++) {
-        if (t < nb) {
-          const float4 a = R.a[4 * t + r];
-          const float4 d = win[cols[t] - w.x];
-          float tt = __fmul_rn(a.x, d.x);
-          tt = __fmaf_rn(a.y, d.y, tt);
-          tt = __fmaf_rn(a.z, d.z, tt);
-          tt = __fmaf_rn(a.w, d.w, tt);
-          acc = __fsub_rn(acc, tt);
-        }
-      }
-      const float b0 = __shfl_sync(qmask, acc, qbase);
-      const float b1 = __shfl_sync(qmask, acc, qbase + 1);
-      const float b2 = __shfl_sync(qmask, acc, qbase + 2);
-      const float b3 = __shfl_sync(qmask, acc, qbase + 3);
-      if (r == 0) {
-        const float4 M0 = R.lu[0], M1 = R.lu[1], M2 = R.lu[2], M3 = R.lu[3];
-        const float y0 = b0;
-        const float y1 = __fmaf_rn(-M1.x, y0, b1);
-        const float y2 = __fmaf_rn(-M2.y, y1, __fmaf_rn(-M2.x, y0, b2));
-        const float y3 = __fmaf_rn(-M3.z, y2, __fmaf_rn(-M3.y, y1, __fmaf_rn(-M3.x, y0, b3)));
-        const float x3 = __fmul_rn(y3, M3.w);
-        const float x2 = __fmul_rn(__fmaf_rn(-M2.w, x3, y2), M2.z);
-        const float x1 = __fmul_rn(__fmaf_rn(-M1.w, x3, __fmaf_rn(-M1.z, x2, y1)), M1.y);
-        const float x0 = __fmul_rn(
-            __fmaf_rn(-M0.w, x3, __fmaf_rn(-M0.z, x2, __fmaf_rn(-M0.y, x1, y0))), M0.x);
-        const float4 x = make_float4(x0, x1, x2, x3);
-        win[j - w.x] = x;
-        X[j] = x;
-        if (last) reinterpret_cast<double4*>(s.dQ)[j] = make_double4(x0, x1, x2, x3);
-      }
-    }
-    // one barrier per sub-level: this level's results are visible to the
-    // next, and the next level's records (all but the newest SLOTS-2 copy
-    // groups) have landed
-    cp_async_wait<SLOTS - 2>();
-    __syncthreads();
+    for (int t = 0; t < kRecBlocks; t++)
+      if (t < nb) c[t] = (unsigned)(ja[k0 + t] - w0);
+    h = slot_info(j - w0, nb, info.y);
   }
-  cp_async_wait<0>();
+  cols[i] = make_uint4(c[0] | c[1] << 16, c[2] | c[3] << 16, c[4] | c[5] << 16, c[6] | c[7] << 16);
+  rows[i] = h;
 }
 
-template <int DIR, int ROWS>
-__global__ void __launch_bounds__(256) k_sweep_chunk(DevState s, ChunkTables ct, float* dq32,
-                                                     int colour, int last) {
+__device__ __forceinline__ void level_init(unsigned long long* bar, unsigned count) {
+  asm volatile("mbarrier.init.shared.b64 [%0], %1;" ::"r"(
+                   static_cast<uint32_t>(__cvta_generic_to_shared(bar))),
+               "r"(count)
+               : "memory");
+}
+__device__ __forceinline__ void level_arrive(unsigned long long* bar) {
+  asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(
+                   static_cast<uint32_t>(__cvta_generic_to_shared(bar)))
+               : "memory");
+}
+// Wait for the barrier's phase of this parity, at most kLevelTries tries (a
+// try itself waits a while in hardware); 0 when they run out.  The loop is
+// written in PTX so that its branches are uniform: the caller's exchanges
+// between lanes then need no reconvergence of the warp.
+constexpr int kLevelTries = 1 << 16;
+__device__ __forceinline__ int level_wait(unsigned long long* bar, unsigned parity) {
+  int left = kLevelTries;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "LEVEL_TRY:\n\t"
+      "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\t"
+      "@p bra.uni LEVEL_DONE;\n\t"
+      "sub.s32 %0, %0, 1;\n\t"
+      "setp.gt.s32 q, %0, 0;\n\t"
+      "@q bra.uni LEVEL_TRY;\n\t"
+      "LEVEL_DONE:\n\t}"
+      : "+r"(left)
+      : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(bar))), "r"(parity)
+      : "memory");
+  return left;
+}
+
+// A chunk's levels in shared memory: one mbarrier each that counts the
+// level's tiles (a phase per pass over the chunk).
+struct ChunkView {
+  int w0;           // the row of window position 0: one before the window's first
+  int nlev;         // levels
+  int t0, ntile;    // the chunk's tiles
+};
+
+template <int WARPS>
+__device__ __forceinline__ ChunkView chunk_levels(const ChunkTables& ct, int q,
+                                                  unsigned long long* bars) {
+  ChunkView v;
+  v.w0 = ct.window[q].x - 1;
+  const int l0 = ct.chunk_lev[q];
+  v.nlev = min(ct.chunk_lev[q + 1] - l0, kChunkSubMax);
+  v.t0 = ct.lev_tile[l0];
+  v.ntile = ct.lev_tile[l0 + v.nlev] - v.t0;
+  for (int i = threadIdx.x; i < v.nlev; i += 32 * WARPS)
+    level_init(bars + i, (unsigned)(ct.lev_tile[l0 + i + 1] - ct.lev_tile[l0 + i]));
+  return v;
+}
+
+template <int WARPS>
+__device__ __forceinline__ void chunk_window(const ChunkTables& ct, int q, const float* dq32) {
+  extern __shared__ __align__(16) float4 sweep_win[];
+  const int2 w = ct.window[q];
+  const float4* X = reinterpret_cast<const float4*>(dq32) + w.x - 1;
+  if (threadIdx.x == 0) sweep_win[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int i = threadIdx.x + 1; i <= w.y - w.x + 1; i += 32 * WARPS) cp_async16(sweep_win + i, X + i);
+  cp_async_commit();
+}
+
+// Pass number `pass` of the CTA over its chunk, DIR 0 forward, 1 backward.
+// ready() returns once the window is in shared memory and the level barriers
+// are set, past a barrier of the CTA.  store: write the rows' results to the
+// iterate (off for a pass that the same CTA's next pass overwrites); last:
+// also to the FP64 dQ.
+template <int DIR, int LANES, int WARPS, class Ready>
+__device__ __forceinline__ void sweep_chunk_pass(const DevState& s, const ChunkTables& ct,
+                                                 float* dq32, const ChunkView& v,
+                                                 unsigned long long* bars, int pass, bool store,
+                                                 int last, Ready&& ready) {
+  extern __shared__ __align__(16) float4 sweep_win[];
+  constexpr int R = tile_rows(LANES), PER = 4 / LANES;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  auto tile_at = [&](int k) { return DIR == 0 ? v.t0 + k : v.t0 + v.ntile - 1 - k; };
+  bool timeout = false;
+  unsigned h = 0, hn = 0;
+  uint4 c = make_uint4(0, 0, 0, 0), cn = c;
+  float4 a[kRecBlocks][PER], m0, m1, m2, m3;
+  float rhs[PER];
+  m0 = m1 = m2 = m3 = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < PER; i++) {
+    rhs[i] = 0.f;
+#pragma unroll
+    for (int t = 0; t < kRecBlocks; t++) a[t][i] = m0;
+  }
+  auto load_row = [&](int k, unsigned& hh, uint4& cc) {
+    if (k < v.ntile) {
+      const int i = R * tile_at(k) + lane / LANES;
+      hh = ct.rows[i];
+      cc = ct.cols[i];
+    }
+  };
+  // blocks and factors of tile k, whose rows are hh
+  auto load_tile = [&](int k, unsigned hh) {
+    if (k < v.ntile) {
+      const float4* T = ct.tiles + (long)tile_at(k) * tile_words(LANES);
+      const int nb = slot_blocks(hh);
+#pragma unroll
+      for (int t = 0; t < kRecBlocks; t++)
+#pragma unroll
+        for (int i = 0; i < PER; i++)
+          a[t][i] = t < nb ? __ldcg(T + 32 * (PER * t + i) + lane)
+                           : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (lane < R) {
+        m0 = __ldcg(T + 32 * R + lane);
+        m1 = __ldcg(T + 33 * R + lane);
+        m2 = __ldcg(T + 34 * R + lane);
+        m3 = __ldcg(T + 35 * R + lane);
+      }
+      const float* b = reinterpret_cast<const float*>(T + 36 * R) + PER * lane;
+      if (PER == 2) {
+        const float2 f = __ldcg(reinterpret_cast<const float2*>(b));
+        rhs[0] = f.x; rhs[PER - 1] = f.y;
+      } else {
+        rhs[0] = __ldcg(b);
+      }
+    }
+  };
+  int k = __shfl_sync(FULL, (int)threadIdx.x >> 5, 0);  // uniform in the warp
+  load_row(k, h, c);
+  load_row(k + WARPS, hn, cn);
+  load_tile(k, h);
+  ready();
+  for (; k < v.ntile; k += WARPS) {
+    const float4* d[kRecBlocks] = {
+        sweep_win + (c.x & 0xffff), sweep_win + (c.x >> 16), sweep_win + (c.y & 0xffff),
+        sweep_win + (c.y >> 16),    sweep_win + (c.z & 0xffff), sweep_win + (c.z >> 16),
+        sweep_win + (c.w & 0xffff), sweep_win + (c.w >> 16)};
+    // the row lane < R solves, and the tile's level
+    const unsigned hs = __shfl_sync(FULL, h, LANES * lane);
+    const bool row = (hs >> 31) && lane < R;
+    const int pos = slot_pos(hs);
+    const int lev = __shfl_sync(FULL, slot_level(h), 0);
+    if (DIR == 0 ? lev > 0 : lev < v.nlev - 1)
+      timeout |= !level_wait(bars + (DIR == 0 ? lev - 1 : lev + 1), pass & 1);
+    float tt[kRecBlocks][PER];
+#pragma unroll
+    for (int t = 0; t < kRecBlocks; t++) {
+      const float4 x = *d[t];
+#pragma unroll
+      for (int i = 0; i < PER; i++) {
+        tt[t][i] = __fmul_rn(a[t][i].x, x.x);
+        tt[t][i] = __fmaf_rn(a[t][i].y, x.y, tt[t][i]);
+        tt[t][i] = __fmaf_rn(a[t][i].z, x.z, tt[t][i]);
+        tt[t][i] = __fmaf_rn(a[t][i].w, x.w, tt[t][i]);
+      }
+    }
+    // an unused block's product is +0, and acc - 0 is acc, whatever its sign
+    float acc[PER];
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+      acc[i] = rhs[i];
+#pragma unroll
+      for (int t = 0; t < kRecBlocks; t++) acc[i] = __fsub_rn(acc[i], tt[t][i]);
+    }
+    // row r's sum is in lane LANES w + r / PER, its sum r % PER
+    const float y0 = __shfl_sync(FULL, acc[0], LANES * lane);
+    const float b1 = __shfl_sync(FULL, acc[1 % PER], LANES * lane + 1 / PER);
+    const float b2 = __shfl_sync(FULL, acc[2 % PER], LANES * lane + 2 / PER);
+    const float b3 = __shfl_sync(FULL, acc[3 % PER], LANES * lane + 3 / PER);
+    const float y1 = __fmaf_rn(-m1.x, y0, b1);
+    const float y2 = __fmaf_rn(-m2.y, y1, __fmaf_rn(-m2.x, y0, b2));
+    const float y3 = __fmaf_rn(-m3.z, y2, __fmaf_rn(-m3.y, y1, __fmaf_rn(-m3.x, y0, b3)));
+    const float x3 = __fmul_rn(y3, m3.w);
+    const float x2 = __fmul_rn(__fmaf_rn(-m2.w, x3, y2), m2.z);
+    const float x1 = __fmul_rn(__fmaf_rn(-m1.w, x3, __fmaf_rn(-m1.z, x2, y1)), m1.y);
+    const float x0 =
+        __fmul_rn(__fmaf_rn(-m0.w, x3, __fmaf_rn(-m0.z, x2, __fmaf_rn(-m0.y, x1, y0))), m0.x);
+    const float4 x = make_float4(x0, x1, x2, x3);
+    if (row) sweep_win[pos] = x;
+    __syncwarp();
+    if (lane == 0) level_arrive(bars + lev);
+    // off the chain: the next tile's loads, this row's results to memory
+    load_tile(k + WARPS, hn);
+    h = hn;
+    c = cn;
+    load_row(k + 2 * WARPS, hn, cn);
+    if (row) {
+      const int j = v.w0 + pos;
+      if (store) reinterpret_cast<float4*>(dq32)[j] = x;
+      if (last) reinterpret_cast<double4*>(s.dQ)[j] = make_double4(x0, x1, x2, x3);
+    }
+  }
+  if (timeout && lane == 0) atomicOr(s.status, ERR_SWEEP_TIMEOUT);
+}
+
+// The register cap: 16 warps' worth of 128 registers, shared by as many CTAs
+// as that makes (small chunks and other solves share the SM).
+template <int DIR, int LANES, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, ring_warps(0) / WARPS)
+    k_sweep_chunk(DevState s, ChunkTables ct, float* dq32, int colour, int last) {
   if (*s.stop) return;  // the run has converged
   const int q = ct.col_chunks[ct.col_ptr[colour] + blockIdx.x];
-  __shared__ int ss[kChunkSubMax + 1];
-  sweep_chunk_body<DIR, ROWS, false>(s, ct, dq32, q, last, ss, [] {});
+  __shared__ unsigned long long bars[kChunkSubMax];
+  chunk_window<WARPS>(ct, q, dq32);
+  const ChunkView v = chunk_levels<WARPS>(ct, q, bars);
+  sweep_chunk_pass<DIR, LANES, WARPS>(s, ct, dq32, v, bars, 0, true, last, [] {
+    cp_async_wait<0>();
+    __syncthreads();
+  });
 }
 
 // Two passes of one colour back to back: the DIR pass of a sweep (it ends
@@ -1863,15 +1985,21 @@ __global__ void __launch_bounds__(256) k_sweep_chunk(DevState s, ChunkTables ct,
 // and no other colour runs between the two passes, so each chunk sweeps
 // itself twice with its window kept in shared memory: what two launches
 // compute, with one launch, one window load and no barrier between them.
-template <int DIR, int ROWS>
-__global__ void __launch_bounds__(256) k_sweep_chunk_pair(DevState s, ChunkTables ct,
-                                                          float* dq32, int colour, int last) {
+template <int DIR, int LANES, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, ring_warps(0) / WARPS)
+    k_sweep_chunk_pair(DevState s, ChunkTables ct, float* dq32, int colour, int last) {
   if (*s.stop) return;  // the run has converged
   const int q = ct.col_chunks[ct.col_ptr[colour] + blockIdx.x];
-  __shared__ int ss[kChunkSubMax + 1];
-  sweep_chunk_body<DIR, ROWS, false>(s, ct, dq32, q, 0, ss, [] {});
-  __syncthreads();  // the first pass's window is complete before the second reads it
-  sweep_chunk_body<1 - DIR, ROWS, false>(s, ct, dq32, q, last, ss, [] {}, true);
+  __shared__ unsigned long long bars[kChunkSubMax];
+  chunk_window<WARPS>(ct, q, dq32);
+  const ChunkView v = chunk_levels<WARPS>(ct, q, bars);
+  sweep_chunk_pass<DIR, LANES, WARPS>(s, ct, dq32, v, bars, 0, false, 0, [] {
+    cp_async_wait<0>();
+    __syncthreads();
+  });
+  // every row of the first pass is in the window before the second begins
+  sweep_chunk_pass<1 - DIR, LANES, WARPS>(s, ct, dq32, v, bars, 1, true, last,
+                                          [] { __syncthreads(); });
 }
 
 // A whole mode 3 sweep in one launch (one CTA per chunk): CTAs take chunks
@@ -1888,8 +2016,8 @@ __global__ void __launch_bounds__(256) k_sweep_chunk_pair(DevState s, ChunkTable
 // stores generation + 1 in ct.done.  A wait gives up after max_spin polls,
 // sets FLOW_ERR_SWEEP_TIMEOUT and goes on (the chunk still finishes, so the
 // counters stay consistent).
-template <int DIR>
-__global__ void __launch_bounds__(256) k_sweep_chunk_df(DevState s, ChunkTables ct,
+template <int DIR, int LANES>
+__global__ void __launch_bounds__(32 * ring_warps(0)) k_sweep_chunk_df(DevState s, ChunkTables ct,
                                                         float* dq32, int last, long max_spin) {
   if (*s.stop) return;  // the run has converged (every CTA of the launch sees it)
   __shared__ int task_q, task_gen;
@@ -1925,8 +2053,15 @@ __global__ void __launch_bounds__(256) k_sweep_chunk_df(DevState s, ChunkTables 
     }
     __syncthreads();
   };
-  __shared__ int ss[kChunkSubMax + 1];
-  sweep_chunk_body<DIR, 64, true>(s, ct, dq32, q, last, ss, wait_deps);
+  __shared__ unsigned long long bars[kChunkSubMax];
+  const ChunkView v = chunk_levels<ring_warps(0)>(ct, q, bars);
+  // the first tiles are loaded before the wait, the window after it
+  sweep_chunk_pass<DIR, LANES, ring_warps(0)>(s, ct, dq32, v, bars, 0, true, last, [&] {
+    wait_deps();
+    chunk_window<ring_warps(0)>(ct, q, dq32);
+    cp_async_wait<0>();
+    __syncthreads();
+  });
   // publish: every thread's iterate writes before the chunk's flag
   __threadfence();
   __syncthreads();

@@ -84,30 +84,34 @@ struct MixedTables {
 // into chunks of consecutive rows (at most a set number of rows and of
 // dependency levels each), coloured greedily so that chunks of one colour
 // share no block; a sweep runs the colours in order, one CTA per chunk, and
-// inside a chunk the rows in the reference's order, level by level.  Each
-// direction keeps one record per row, in chunk / sub-level order, with all
-// the sweep reads of that row; a sub-level is at most kRecRows rows of one
-// level.
-constexpr int kRecBlocks = 8;  // off-diagonal blocks a record holds
-
-struct __align__(16) SweepRec {
-  int4 hdr;                 // row j, off-diagonal block count, 0, 0
-  float4 rhs;               // right-hand side (FP32)
-  float4 lu[4];             // LU factors of the diagonal block, reciprocal pivots
-  int4 cols[2];             // columns of the off-diagonal blocks (0: none)
-  float4 a[4 * kRecBlocks]; // the blocks, row-major, block t row r at a[4t + r]
-};
+// inside a chunk the rows in the reference's order, level by level: forward
+// sweeps take the levels ascending, backward ones descending (of two
+// adjacent rows the later one has the higher level, so either way a row runs
+// after the neighbours its sweep updates first).  The rows of a level are
+// dealt R = 32 / lanes to a tile, the last tile of a level padded with empty
+// slots; a warp takes a tile, `lanes` (4 or 2) of its lanes a row, and every
+// load of the warp from a tile is contiguous.  A tile in float4 words,
+// w the row's slot in it:
+//   row r of block t     32 (4 / lanes * t + r % (4 / lanes)) + lanes w + r / (4 / lanes)
+//   row r of the factors 32 R + R r + w   (LU of the diagonal block, reciprocal pivots)
+//   right-hand side      36 R + w         (FP32)
+constexpr int kRecBlocks = 8;  // off-diagonal blocks a row of a tile holds
+__host__ __device__ constexpr int tile_rows(int lanes) { return 32 / lanes; }
+__host__ __device__ constexpr int tile_words(int lanes) { return 37 * tile_rows(lanes); }
 
 struct ChunkTables {
   int nchunks, ncol, maxwin;
   const int* col_ptr;        // ncol+1: chunks of each colour in col_chunks
   const int* col_chunks;
   const int2* window;        // per chunk: first and last row any of its rows touches
-  SweepRec* rec[2];          // per direction (0 forward, 1 backward)
-  const int* sub_start[2];   // record index of each sub-level, plus the end
-  const int* chunk_sub[2];   // first sub-level of each chunk, plus the end
-  const int* pos[2];         // record index of each row (1..nn)
-  int ring;                  // ring shape of the sub-level tables: rows 64 >> ring
+  float4* tiles;             // chunk by chunk, level by level
+  int lanes_log2;            // lanes a row of a tile takes: 1 << lanes_log2
+  const uint4* cols;         // per slot: the blocks' columns as 16-bit window positions
+  const unsigned* rows;      // per slot: its row, block count and level (slot_info), 0: empty
+  const int* lev_tile;       // first tile of each level, plus the end
+  const int* chunk_lev;      // first level of each chunk, plus the end
+  const int* slot;           // slot of each row (1..nn)
+  int ring;                  // CTA shape of the sweep (ring_warps)
   // one-launch (dataflow) sweeps
   const int* task_chunk[2];  // per direction: chunks in dispensing (colour) order
   const int* colour;         // colour of each chunk

@@ -593,7 +593,7 @@ class Solver:
         _check(self.L.flow_set_chunk(self.ctx, int(rows), int(levels)), "flow_set_chunk")
 
     def set_sweep_ring(self, rows: int = 0):
-        """Sub-level rows of the mode 3 sweep's prefetch ring (64, 32, 16)."""
+        """CTA shape of the mode 3 sweep: 64, 32 or 16 for 16, 8 or 4 warps."""
         _check(self.L.flow_set_sweep_ring(self.ctx, int(rows)), "flow_set_sweep_ring")
 
     def set_sweep_dataflow(self, on: bool = True):

@@ -67,11 +67,12 @@ def ordered_sweep_bytes(mesh) -> int:
 
 def chunk_sweep_bytes(mesh) -> int:
     """One whole chunked FP32 sweep (precision mode 3, all colour launches):
-    per row its 640-byte sweep record (header, right-hand side, LU factors,
-    8 columns, 8 FP32 blocks) staged once, its iterate read through the
-    chunk's window and written back (16 + 16)."""
+    per row its factors and right-hand side 80, window positions and row word
+    20, its iterate read through the chunk's window and written back (16 +
+    16); per off-diagonal block its FP32 values 64."""
     z = _sizes(mesh)
-    return int(z["nn"] * (640 + 16 + 16))
+    offd = z["nnz"] - z["nn"]
+    return int(z["nn"] * (80 + 20 + 32) + offd * 64)
 
 
 def subedge_flux_bytes(mesh, jacobian: bool = True, approx: bool = False) -> int:
@@ -91,13 +92,14 @@ def assemble_bytes(mesh, precision: int = 3, approx: bool = False) -> int:
     face's flux 32 and Jacobian block J read; per off-diagonal block its
     subedge pair 16 and the one or two face Jacobians (two a block on these
     meshes) 2J read; per node dt, cv_area 16 read, R and RHS 64 written and
-    its row written: two 640-byte sweep records (mode 3), or FP64 blocks
-    128 a block and LU factors 128 (mode 0).  J = 128 (FP64) or 64 (the
+    its row written: its FP32 blocks 64 a block, factors and right-hand side
+    80 (mode 3), or FP64 blocks 128 a block and LU factors 128 (mode 0).  J = 128 (FP64) or 64 (the
     approximate Jacobian's FP32 blocks)."""
     z = _sizes(mesh)
     offd = z["nnz"] - z["nn"]
     J = 64 if approx else 128
-    row = 2 * 640 if precision == 3 else 128 * z["nnz"] / max(z["nn"], 1) + 128
+    nn = max(z["nn"], 1)
+    row = 80 + 64 * offd / nn if precision == 3 else 128 * z["nnz"] / nn + 128
     return int(2 * z["ns"] * (4 + 32 + J) + offd * (16 + 2 * J) + z["nn"] * (16 + 64 + row))
 
 
@@ -106,8 +108,9 @@ def faces_assemble_bytes(mesh) -> int:
     incidence its entry and block slot 8, the face's end nodes 8,
     normal/length 32 and the other node's state 32 read (k=1: the two nodes'
     gradients and limiters 144 and the offsets 32); per node its own state
-    32, dt and cv_area 16, R and RHS 64 and its two 640-byte sweep records;
-    per boundary edge its flux and Jacobian 160 read."""
+    32, dt and cv_area 16, R and RHS 64, and its row's factors, right-hand
+    side and blocks 80 + 64 a block; per boundary edge its flux and Jacobian 160 read."""
     z = _sizes(mesh)
     per_inc = 8 + 8 + 32 + 32 + (0 if mesh.order == 3 else 144 + 32)
-    return int(2 * z["ns"] * per_inc + z["nn"] * (32 + 16 + 64 + 2 * 640) + z["nbe"] * 160)
+    offd = z["nnz"] - z["nn"]
+    return int(2 * z["ns"] * per_inc + z["nn"] * (32 + 16 + 64 + 80) + offd * 64 + z["nbe"] * 160)

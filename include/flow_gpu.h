@@ -340,19 +340,19 @@ int flow_set_sweep_pairs(flow_ctx *ctx, int on);
 /* Chunk limits of precision mode 3 (0: defaults, rows = twice the matrix
  * bandwidth up to 2048, levels = 32). */
 int flow_set_chunk(flow_ctx *ctx, int rows, int levels);
-/* Ring shape of the mode 3 sweep (no counterpart in the reference): the
- * records of sub-levels of `rows` rows (64, 32 or 16; 0 = 64) are prefetched
- * into a shared-memory ring of 3, 6 or 12 slots.  Rows of one dependency
- * level are independent, so every shape gives the same results; smaller
- * sub-levels prefetch further ahead.  FLOW_ERR_ARG (shape unchanged) if a
- * chunk would hold more sub-levels than the sweep kernel does. */
+/* CTA shape of the mode 3 sweep (no counterpart in the reference): `rows` 64,
+ * 32 or 16 (0 = 64) names a sweep CTA of 16, 8 or 4 warps; more warps keep
+ * more rows in flight, fewer leave room for other chunks.  Rows of one
+ * dependency level are independent, so every shape gives the same results.
+ * FLOW_ERR_ARG (shape unchanged) if a chunk's levels, cut into runs of that
+ * many rows, make more than 256 runs. */
 int flow_set_sweep_ring(flow_ctx *ctx, int rows);
 /* One-launch mode 3 sweeps (no counterpart in the reference): on != 0 runs
  * each sweep as one launch in which a chunk starts as soon as the chunks of
  * earlier colours that its window overlaps have finished, instead of one
  * launch per colour; the same results (each chunk reads its neighbours at
  * the same point of the sweep).  Waits are bounded: one that runs out sets
- * FLOW_ERR_SWEEP_TIMEOUT.  Used with the 64-row ring shape. */
+ * FLOW_ERR_SWEEP_TIMEOUT.  Used with the 64-row shape. */
 int flow_set_sweep_dataflow(flow_ctx *ctx, int on);
 /* Mode 3 chunks in use: starts[0..nchunks] (first row of each chunk, then
  * nn+1; up to cap entries written), their number and the colour count. */
@@ -448,12 +448,12 @@ int flow_autotune(flow_ctx *ctx, const flow_params *p, int ts, int steps, int *v
                   double *ms);
 int flow_set_variants(flow_ctx *ctx, int node_prepare, int flux);
 /* The sweep of precision mode 3 in the shape that runs fastest on this mesh:
- * the record ring of 64, 32 or 16-row sub-levels with one launch per colour
- * (colours per launch = 1), and, with allow_df, the 64-row ring with the
+ * CTAs of 16, 8 or 4 warps (flow_set_sweep_ring 64, 32, 16) with one launch per
+ * colour (colours per launch = 1), and, with allow_df, 16 warps with the
  * whole sweep in one launch (flow_set_sweep_dataflow; its chunks wait for
  * their neighbours on the device, so among many solves it holds SMs that
  * others could use).  Every shape gives the same bits.  Timed like
- * flow_autotune, the state put back; *choice = the rows of the chosen ring,
+ * flow_autotune, the state put back; *choice = the rows naming the chosen shape,
  * plus 1000 for one launch per sweep; ms[4] (may be NULL) the sweep times
  * (1e30 where a shape does not fit or is not allowed).  The sweep count is
  * not chosen here: it changes the iterates, not only their speed. */
