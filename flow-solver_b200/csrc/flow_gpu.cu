@@ -184,6 +184,7 @@ struct flow_ctx {
   // one-CTA ordered sweep: stage tables (null when the matrix bandwidth is too
   // large for its dQ window, then the multi-CTA sweep is used)
   SweepTables sweep_tb{};
+  LevelTables levels{};  // FP64 sweep by levels (build_levels); nlev 0: not used
   bool sweep_cta_ok = false;
   double* d_hist = nullptr;  // 2 x hist_cap device history of (dq, r_rho)
   int hist_cap = 0;
@@ -381,6 +382,7 @@ constexpr int kVariants = 3;
 // and by no zero (venkat_fold_nz), variant 5 with the wave-speed face terms
 // in the limiter's face loop too (LIM = 2; variants 6 and 7 LIM = 1).
 constexpr int kNodeVariants = 8;
+constexpr int kLevelSmemMax = 227 * 1024;  // k_sweep_levels
 constexpr size_t kStageSmemMax = 110 * 1024;  // two CTAs per SM at most
 template <class F>
 void launch_variant(int v, F&& f) {
@@ -660,7 +662,6 @@ int launch_linear_solve(flow_ctx* c, const flow_params* p, bool final_rms) {
   cudaMemsetAsync(c->s.skip, 0, sizeof(int), c->stream);
   const long max_spin = 1L << 21;  // ~0.1-0.2 s per wait at most
   for (int it = 0; it < p->subits; it++) {
-    cudaMemsetAsync(c->s.counter, 0, sizeof(unsigned), c->stream);
     {
       Timed t(c, 4);
       if (c->sweep_cta_ok && c->sweep_mode == 1) {
@@ -670,9 +671,17 @@ int launch_linear_solve(flow_ctx* c, const flow_params* p, bool final_rms) {
         else
           k_sweep_cta<false><<<1, kSweepThreads, sm, c->stream>>>(c->m, c->s, c->sweep_tb, max_spin);
         rc |= launch_check(c);
+      } else if (c->levels.nlev > 0) {
+        const size_t sm = level_smem_bytes(c->levels.nlev, c->levels.ring);
+        if (it % 2 == 0)
+          k_sweep_levels<true><<<1, kLevelThreads, sm, c->stream>>>(c->m, c->s, c->levels, it == 0);
+        else
+          k_sweep_levels<false><<<1, kLevelThreads, sm, c->stream>>>(c->m, c->s, c->levels, 0);
+        rc |= launch_check(c);
       } else {
         // results go to the other dQ buffer, pre-filled with the not-ready
         // pattern; the buffers swap roles afterwards
+        cudaMemsetAsync(c->s.counter, 0, sizeof(unsigned), c->stream);
         double* dq_new = c->s.dQ2;
         k_prepare_sweep<<<grid_blocks(4 * (c->nn + 1), 256), 256, 0, c->stream>>>(
             c->s, c->s.dQ, dq_new, 4 * (c->nn + 1));
@@ -802,7 +811,7 @@ int enqueue_chunk(flow_ctx* c, const flow_params* p, int ts0, int K) {
   const bool graphable = c->use_graphs && !c->timing && K > 0 && ph == phase_of(p, ts0 + K - 1) &&
                          sw == sweeps_at(c, p, ts0 + K - 1) &&
                          (c->precision == 1 || c->precision == 3 ||
-                          (c->precision == 0 && c->sweep_mode == 1) ||
+                          (c->precision == 0 && (c->sweep_mode == 1 || c->levels.nlev > 0)) ||
                           p->subits % 2 == 0);
   if (!graphable) {
     for (int i = 0; i < K && !rc; i++) rc |= enqueue_step(c, p, ts0 + i, -1, -1, true);
@@ -1054,11 +1063,127 @@ bool ensure_kernel_attrs(int device) {
                         (const void*)k_faces_assemble<0, 2>, (const void*)k_faces_assemble<1, 2>})
     ok = ok && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)kFusedSmem) == cudaSuccess;
+  for (const void* f : {(const void*)k_sweep_levels<true>, (const void*)k_sweep_levels<false>})
+    ok = ok && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kLevelSmemMax) ==
+                   cudaSuccess;
   for (const void* f : {(const void*)k_sweep_cta<true>, (const void*)k_sweep_cta<false>})
     ok = ok && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, cta) ==
                    cudaSuccess;
   if (ok) done[device] = 1;
   return ok;
+}
+
+// Tables of k_sweep_levels, where the matrix suits it: at most kRecBlocks
+// off-diagonal blocks a row with the diagonal block last, levels that are not
+// too wide, and a window of dQ that fits in shared memory.  Otherwise, and
+// where the tables find no room, the context keeps the grid-wide sweep.
+void build_levels(flow_ctx* c) {
+  if (c->levels.nlev > 0) return;
+  const int nn = c->nn;
+  const std::vector<int>& ia = c->h_ia;
+  const std::vector<int>& ja = c->h_ja;
+  std::vector<int> lev(nn + 1, 0);
+  int nlev = 0;
+  for (int j = 1; j <= nn; j++) {
+    const int nb = ia[j + 1] - ia[j] - 1;
+    if (nb < 0 || nb > kRecBlocks || ja[ia[j + 1] - 1] != j) return;
+    int l = 0;
+    for (int k = ia[j]; k < ia[j] + nb; k++)
+      if (ja[k] < j) l = std::max(l, lev[ja[k]] + 1);
+    lev[j] = l;
+    nlev = std::max(nlev, l + 1);
+  }
+  if (nlev > kLevelMax || nn > (long)kLevelWidthMax * nlev) return;
+  // tiles and positions: level by level, rows ascending
+  std::vector<int> count(nlev + 1, 0), lev_tile(nlev + 1, 0), pos(nn + 1, 0);
+  for (int j = 1; j <= nn; j++) count[lev[j] + 1]++;
+  for (int l = 0; l < nlev; l++) {
+    lev_tile[l + 1] = lev_tile[l] + (count[l + 1] + 7) / 8;
+    count[l + 1] += count[l];
+  }
+  {
+    std::vector<int> at(count.begin(), count.end() - 1);
+    for (int j = 1; j <= nn; j++) pos[j] = at[lev[j]]++;
+  }
+  // positions a level touches (its rows and their columns)
+  std::vector<int> first(nlev, nn), last(nlev, -1);
+  for (int j = 1; j <= nn; j++) {
+    int lo = nn, hi = -1;
+    for (int k = ia[j]; k < ia[j + 1]; k++) {
+      lo = std::min(lo, pos[ja[k]]);
+      hi = std::max(hi, pos[ja[k]]);
+    }
+    first[lev[j]] = std::min(first[lev[j]], lo);
+    last[lev[j]] = std::max(last[lev[j]], hi);
+  }
+  // per direction (its levels in running order): the positions that must be in
+  // the window before each level, and the smallest ring in which none is
+  // overwritten before the levels that read the old one are done
+  std::vector<int> to[2] = {std::vector<int>(nlev), std::vector<int>(nlev)};
+  int ring = 1;
+  for (int dir = 0; dir < 2; dir++) {
+    std::vector<int> back(nlev);  // the farthest position that level o or a later one touches
+    for (int o = 0; o < nlev; o++) {
+      const int l = dir == 0 ? o : nlev - 1 - o;
+      to[dir][o] = dir == 0 ? std::max(o > 0 ? to[0][o - 1] : 0, last[l] + 1)
+                            : std::min(o > 0 ? to[1][o - 1] : nn, first[l]);
+    }
+    for (int o = nlev - 1; o >= 0; o--) {
+      const int l = dir == 0 ? o : nlev - 1 - o;
+      back[o] = dir == 0 ? first[l] : last[l];
+      if (o + 1 < nlev)
+        back[o] = dir == 0 ? std::min(back[o], back[o + 1]) : std::max(back[o], back[o + 1]);
+    }
+    // while the rows for level o are loaded, levels from o - kLevelsAhead on may run
+    for (int o = 0; o < nlev; o++) {
+      const int b = back[std::max(0, o - kLevelsAhead)];
+      ring = std::max(ring, dir == 0 ? to[0][o] - b : b - to[1][o] + 1);
+    }
+  }
+  if (ring >= 65535 || level_smem_bytes(nlev, ring) > (size_t)kLevelSmemMax) return;
+  std::vector<LevelSlot> slots(8 * (size_t)lev_tile[nlev]);
+  LevelSlot empty{};
+  empty.cols = make_uint4(ring * 65537u, ring * 65537u, ring * 65537u, ring * 65537u);
+  for (int l = 0; l < nlev; l++) {
+    empty.level_nb = (unsigned)l;
+    std::fill(slots.begin() + 8 * (size_t)lev_tile[l], slots.begin() + 8 * (size_t)lev_tile[l + 1],
+              empty);
+  }
+  for (int j = 1; j <= nn; j++) {
+    const int l = lev[j], nb = ia[j + 1] - ia[j] - 1;
+    LevelSlot& S = slots[8 * (size_t)lev_tile[l] + (pos[j] - count[l])];
+    S.row = j;
+    S.block = ia[j];
+    S.level_nb = (unsigned)l | (unsigned)nb << 28;
+    S.pos = pos[j];
+    unsigned q[kRecBlocks];
+    for (int t = 0; t < kRecBlocks; t++)
+      q[t] = t < nb ? (unsigned)(pos[ja[ia[j] + t]] % ring) : (unsigned)ring;
+    S.cols = make_uint4(q[0] | q[1] << 16, q[2] | q[3] << 16, q[4] | q[5] << 16, q[6] | q[7] << 16);
+  }
+  // one buffer: the slots, then the tiles of each level and the two load lists
+  static_assert(sizeof(LevelSlot) == 2 * sizeof(int4), "LevelSlot layout");
+  const size_t nints = (size_t)(nlev + 1) + 2 * (size_t)nlev;
+  std::vector<LevelSlot> all(slots);
+  all.resize(slots.size() + (4 * nints + sizeof(LevelSlot) - 1) / sizeof(LevelSlot));
+  int* ints = reinterpret_cast<int*>(all.data() + slots.size());
+  std::copy(lev_tile.begin(), lev_tile.end(), ints);
+  std::copy(to[0].begin(), to[0].end(), ints + nlev + 1);
+  std::copy(to[1].begin(), to[1].end(), ints + 2 * nlev + 1);
+  const bool was = c->buf.carve_failed;
+  const LevelSlot* d = upload_vec(c, all);
+  if (!d) {  // no room: the grid-wide sweep
+    c->buf.carve_failed = was;
+    return;
+  }
+  LevelTables lt{};
+  lt.ring = ring;
+  lt.slots = d;
+  lt.lev_tile = reinterpret_cast<const int*>(d + slots.size());
+  lt.load_to[0] = lt.lev_tile + nlev + 1;
+  lt.load_to[1] = lt.lev_tile + 2 * nlev + 1;
+  lt.nlev = nlev;
+  c->levels = lt;
 }
 
 // Mode 3 reads none of the mode 1 / 2 tables: only the FP32 iterate.
@@ -1656,7 +1781,8 @@ static flow_ctx* create_impl(flow_arena* arena, const flow_grid_view* g, const f
   s.pv = c->buf.alloc<double>((size_t)(nn + 1) * 4);
   s.dt = c->buf.alloc<double>((size_t)(nn + 1));
   s.LHS = c->buf.alloc<double>((size_t)nnz * 16);
-  s.LUd = c->buf.alloc<double>((size_t)(nn + 1) * 16);
+  s.LUd = c->buf.alloc<double>((size_t)(nn + 1) * 20);
+  s.LUr = s.LUd + (size_t)(nn + 1) * 16;
   s.xn_bedges = c->buf.alloc<double>((size_t)(nbe + 1) * 3);
   s.F = c->buf.alloc<double>((size_t)(ns + 1) * 4);
   s.JL = c->buf.alloc<double>((size_t)(ns + 1) * 16);
@@ -1714,6 +1840,9 @@ static flow_ctx* create_impl(flow_arena* arena, const flow_grid_view* g, const f
   if (!upload(c, s.xn_bedges, xnb.data(), xnb.size() * 8) ||
       !upload(c, c->xnb0, xnb.data(), xnb.size() * 8))
     return fail(c, FLOW_ERR_CUDA, "upload failed");
+  // an arena's contexts mostly run the precision form: they build the FP64
+  // sweep's tables when they are set to precision 0
+  if (!arena) build_levels(c);
   // the context's own stream only: a device-wide synchronisation here would
   // invalidate a graph capture another thread has open
   if (cudaStreamSynchronize(c->stream) != cudaSuccess)
@@ -1782,6 +1911,10 @@ int flow_set_precision(flow_ctx* c, int mode) {
     int rc = mode == 3 ? build_chunk_iterate(c) : build_mixed_tables(c, mode >= 2);
     if (!rc && mode == 3) rc = build_chunk_tables(c);
     if (rc) return rc;
+  } else if (c->levels.nlev == 0) {
+    cudaStreamSynchronize(c->stream);
+    drop_graphs(c);
+    build_levels(c);
   }
   c->precision = mode;
   return 0;

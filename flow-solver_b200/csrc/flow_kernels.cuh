@@ -925,6 +925,7 @@ __device__ __forceinline__ void assemble_row(const DevMesh& m, const DevState& s
     }
   } else {
     reinterpret_cast<double4*>(s.LUd + 16 * (long)n)[q] = make_double4(o0, o1, o2, o3);
+    s.LUr[4 * (long)n + q] = pivot_recip(q == 0 ? o0 : q == 1 ? o1 : q == 2 ? o2 : o3);
   }
 }
 
@@ -1093,6 +1094,7 @@ __global__ void __launch_bounds__(128) k_boundary_add4(DevMesh m, DevState s) {
   lu4(M);
   reinterpret_cast<double4*>(s.LUd + 16 * (long)n)[q] =
       make_double4(M[4 * q], M[4 * q + 1], M[4 * q + 2], M[4 * q + 3]);
+  s.LUr[4 * (long)n + q] = pivot_recip(M[5 * q]);
 }
 
 // LU factors of every diagonal block (linear_algebra.C:226-246), from an LHS
@@ -1112,6 +1114,8 @@ __global__ void __launch_bounds__(128) k_diag_lu(DevMesh m, DevState s) {
 #pragma unroll
   for (int row = 0; row < 4; row++)
     dst[row] = make_double4(M[4 * row], M[4 * row + 1], M[4 * row + 2], M[4 * row + 3]);
+  reinterpret_cast<double4*>(s.LUr)[n] =
+      make_double4(pivot_recip(M[0]), pivot_recip(M[5]), pivot_recip(M[10]), pivot_recip(M[15]));
 }
 
 // ---------------------------------------------------------------------------
@@ -1323,7 +1327,9 @@ __global__ void __launch_bounds__(128) k_diag_only(DevMesh m, DevState s) {
 }
 
 // ---------------------------------------------------------------------------
-// Ordered block Gauss-Seidel sweep (linear_algebra.C:178-344).  Rows are
+// Ordered block Gauss-Seidel sweep (linear_algebra.C:178-344) over the whole
+// GPU, for matrices whose levels are wide (kLevelWidthMax; k_sweep_levels
+// otherwise).  Rows are
 // handed out in the reference's order (ascending forward, descending
 // backward) by an atomic dispenser; one warp per row.  The sweep writes its
 // results into dq_new, which is filled with an all-ones bit pattern (a NaN
@@ -1335,7 +1341,11 @@ __global__ void __launch_bounds__(128) k_diag_only(DevMesh m, DevState s) {
 // only claimed by running warps and every dependency was claimed earlier,
 // so the earliest unfinished row always proceeds; every wait is nevertheless
 // bounded and reports ERR_SWEEP_TIMEOUT instead of spinning forever.
-// Lanes: 8 block slots x 4 matrix rows.
+// Lanes: 8 block slots x 4 matrix rows; the factors are loaded, by every lane,
+// before the waits, and the solve divides by the pivots' reciprocals (865 ->
+// 805 us a sweep on 65,536 rows, 505 -> 471 on 25,600).  The stores stay one
+// value at a time: a 16-byte relaxed store, or one value a lane picked by a
+// select, made a level three times as long.
 constexpr unsigned long long kNotReady = 0xFFFFFFFFFFFFFFFFull;
 
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const double* p) {
@@ -1346,6 +1356,24 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const double* p) {
 
 __device__ __forceinline__ void st_relaxed_f64(double* p, double v) {
   asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+
+// The four values of a row as one relaxed access (each value is single-copy
+// atomic by itself, which is all the ready pattern needs).
+__device__ __forceinline__ void ld_relaxed_row(const double* p, unsigned long long* u) {
+  for (int i = 0; i < 4; i++) u[i] = ld_relaxed_u64(p + i);
+}
+__device__ __forceinline__ void st_relaxed_row(double* p, const double* v) {
+  for (int i = 0; i < 4; i++) st_relaxed_f64(p + i, v[i]);
+}
+// A double4 in one 32-byte access.
+__device__ __forceinline__ double4 ld_d4(const double* p) {
+  double4 v;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
 }
 
 template <bool FWD>
@@ -1365,23 +1393,22 @@ __global__ void __launch_bounds__(128) k_sweep_ordered(DevMesh m, DevState s,
     if (t >= (unsigned)nn) break;
     const int j = FWD ? (int)(1 + t) : (int)(nn - t);
     const int k0 = m.ia[j], k1 = m.ia[j + 1];
-    // everything that does not depend on this sweep's results first
+    // everything that does not depend on this sweep's results first, the
+    // factors and the row's old value by every lane (each forms the solution)
     double acc = s.RHS[4 * (long)j + r];
-    const double lu_v = (lane < 16) ? s.LUd[16 * (long)j + lane] : 0.;
-    const double old_v = (lane < 4) ? dq_old[4 * (long)j + lane] : 0.;
+    const double4 m0 = ld_d4(s.LUd + 16 * (long)j), m1 = ld_d4(s.LUd + 16 * (long)j + 4);
+    const double4 m2 = ld_d4(s.LUd + 16 * (long)j + 8), m3 = ld_d4(s.LUd + 16 * (long)j + 12);
+    const double4 mr = ld_d4(s.LUr + 4 * (long)j), own = ld_d4(dq_old + 4 * (long)j);
     bool timeout = false;
     for (int base = k0; base < k1; base += 8) {
       const int k = base + slot;
       int c = 0;
       bool use = false;
-      double a0 = 0., a1 = 0., a2 = 0., a3 = 0.;
+      double4 a = make_double4(0., 0., 0., 0.);
       if (k < k1) {
         c = m.ja[k];
         use = c != j;
-        if (use) {
-          const double4 av = reinterpret_cast<const double4*>(s.LHS + 16 * (long)k)[r];
-          a0 = av.x; a1 = av.y; a2 = av.z; a3 = av.w;
-        }
+        if (use) a = ld_d4(s.LHS + 16 * (long)k + 4 * r);
       }
       double term = 0.;
       if (use) {
@@ -1389,14 +1416,12 @@ __global__ void __launch_bounds__(128) k_sweep_ordered(DevMesh m, DevState s,
         double d0, d1, d2, d3;
         if (dep) {
           const double* src = dq_new + 4 * (long)c;
-          unsigned long long u0, u1, u2, u3;
+          unsigned long long u[4];
           long spins = 0;
           for (;;) {
-            u0 = ld_relaxed_u64(src);
-            u1 = ld_relaxed_u64(src + 1);
-            u2 = ld_relaxed_u64(src + 2);
-            u3 = ld_relaxed_u64(src + 3);
-            if (u0 != kNotReady && u1 != kNotReady && u2 != kNotReady && u3 != kNotReady) break;
+            ld_relaxed_row(src, u);
+            if (u[0] != kNotReady && u[1] != kNotReady && u[2] != kNotReady && u[3] != kNotReady)
+              break;
             if (++spins > max_spin) {
               atomicOr(s.status, ERR_SWEEP_TIMEOUT);
               timeout = true;
@@ -1409,46 +1434,37 @@ __global__ void __launch_bounds__(128) k_sweep_ordered(DevMesh m, DevState s,
             }
             if (spins > 256) __nanosleep(32);
           }
-          d0 = __longlong_as_double((long long)u0);
-          d1 = __longlong_as_double((long long)u1);
-          d2 = __longlong_as_double((long long)u2);
-          d3 = __longlong_as_double((long long)u3);
+          d0 = __longlong_as_double((long long)u[0]);
+          d1 = __longlong_as_double((long long)u[1]);
+          d2 = __longlong_as_double((long long)u[2]);
+          d3 = __longlong_as_double((long long)u[3]);
         } else {
           const double2* dq = reinterpret_cast<const double2*>(dq_old + 4 * (long)c);
           const double2 x01 = __ldcg(dq), x23 = __ldcg(dq + 1);
           d0 = x01.x; d1 = x01.y; d2 = x23.x; d3 = x23.y;
         }
-        term = (a0 * d0 + a1 * d1 + a2 * d2 + a3 * d3);
+        term = (a.x * d0 + a.y * d1 + a.z * d2 + a.w * d3);
       }
-      const unsigned used = __ballot_sync(FULL, use);
+      // an unused slot's term is +0, and acc - 0 is acc, whatever its sign
+      __syncwarp();
 #pragma unroll
-      for (int sl = 0; sl < 8; sl++) {
-        double tv = __shfl_sync(FULL, term, sl * 4 + r);
-        if (used & (1u << (sl * 4))) acc -= tv;
-      }
+      for (int sl = 0; sl < 8; sl++) acc -= __shfl_sync(FULL, term, sl * 4 + r);
     }
-    double b[4], M[16], o[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) b[q] = __shfl_sync(FULL, acc, q);
-#pragma unroll
-    for (int q = 0; q < 16; q++) M[q] = __shfl_sync(FULL, lu_v, q);
-#pragma unroll
-    for (int q = 0; q < 4; q++) o[q] = __shfl_sync(FULL, old_v, q);
+    const double b[4] = {__shfl_sync(FULL, acc, 0), __shfl_sync(FULL, acc, 1),
+                         __shfl_sync(FULL, acc, 2), __shfl_sync(FULL, acc, 3)};
+    const double M[16] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w,
+                          m2.x, m2.y, m2.z, m2.w, m3.x, m3.y, m3.z, m3.w};
+    const double rp[4] = {mr.x, mr.y, mr.z, mr.w};
     double X[4];
-    lu_solve4(M, b, X);
-    double mine = X[0], own = o[0];
-#pragma unroll
-    for (int q = 1; q < 4; q++)
-      if (lane == q) { mine = X[q]; own = o[q]; }
+    lu_solve4_recip(M, rp, b, X);
+    // dx = X - dQ, dQ + dx (linear_algebra.C:247-262)
+    double x[4] = {own.x + (X[0] - own.x), own.y + (X[1] - own.y), own.z + (X[2] - own.z),
+                   own.w + (X[3] - own.w)};
     if (__any_sync(FULL, timeout)) {
       // a timed-out row publishes something so that nothing waits on it
-      mine = 0.;
-      own = 0.;
+      x[0] = x[1] = x[2] = x[3] = 0.;
     }
-    if (lane < 4) {
-      const double dx = mine - own;
-      st_relaxed_f64(dq_new + 4 * (long)j + lane, own + dx);
-    }
+    if (lane == 0) st_relaxed_row(dq_new + 4 * (long)j, x);
     __syncwarp();
   }
 }
@@ -1949,11 +1965,14 @@ __device__ __forceinline__ void sweep_chunk_pass(const DevState& s, const ChunkT
     if (row) sweep_win[pos] = x;
     __syncwarp();
     if (lane == 0) level_arrive(bars + lev);
-    // off the chain: the next tile's loads, this row's results to memory
-    load_tile(k + WARPS, hn);
+    // off the chain: the next tile's loads, this row's results to memory.  The
+    // row words move on before the loads are issued (a move behind them could
+    // wait for them)
     h = hn;
     c = cn;
+    asm volatile("" : "+r"(h), "+r"(c.x), "+r"(c.y), "+r"(c.z), "+r"(c.w)::"memory");
     load_row(k + 2 * WARPS, hn, cn);
+    load_tile(k + WARPS, h);
     if (row) {
       const int j = v.w0 + pos;
       if (store) reinterpret_cast<float4*>(dq32)[j] = x;
@@ -2076,6 +2095,191 @@ __global__ void __launch_bounds__(32 * ring_warps(0)) k_sweep_chunk_df(DevState 
       atomicAdd(&ct.sync[2], 1u);
     }
   }
+}
+
+// The FP64 ordered sweep by one CTA: the rows by dependency level, a tile of
+// 8 rows a warp, four lanes a row (lane r owning block row r), a level handed
+// over by an mbarrier that counts its tiles, as in k_sweep_chunk.  dQ is
+// updated in place, kept both by row (s.dQ) and by position in level order
+// (s.dQ2); the CTA keeps a window of the latter in shared memory (a ring; the
+// place after it holds zeros, which unused blocks read).  One more warp loads
+// the window ahead of the levels (kLevelsAhead) and counts as arrivals of the
+// level two before the one that needs the rows; a place of the ring is
+// overwritten only once every level that reads the old one is done (host-checked,
+// build_levels).  fresh: dQ is zero (the first sweep), nothing is loaded.
+//
+// Bound by the chain of levels: the row-by-row sweep over the whole GPU
+// (k_sweep_ordered) pays a publish and a poll through L2 a level, about 925
+// cycles, besides the row's own chain; inside one SM the hand-over takes 110
+// and a level of one or two tiles 1,150 in all (FP64 latency: reads and
+// products 400, the ordered subtraction 60, the 4x4 solve 500).  Wide levels
+// are bound by the tiles one SM works on at a time, and the whole GPU is the
+// faster one: us a sweep, one CTA against k_sweep_ordered, at 11 rows a level
+// (1,024 rows) 52 / 92, at 19 (4,096) 134 / 196, at 33 (10,816) 273 / 306, at
+// 49 (25,600) 638 / 471.  kLevelWidthMax draws the line.  Forming the
+// products with earlier levels' columns before the wait (two blocks a row
+// reloaded or the tile's waiting blocks formed again after it) measured
+// slower: the registers or branches it takes cost more than the chain gains.
+constexpr int kLevelWidthMax = 34;  // mean rows a level
+constexpr int kLevelWarps = 7;      // tiles in flight (255 registers a thread)
+constexpr int kLevelThreads = 32 * (kLevelWarps + 1);
+constexpr int kLevelsAhead = 3;     // levels the window is loaded ahead
+constexpr int kLevelMax = 8192;     // levels (their barriers sit in shared memory)
+
+__host__ __device__ inline size_t level_smem_bytes(int nlev, int ring) {
+  return 32 * ((size_t)ring + 1) + 8 * (size_t)nlev;
+}
+
+template <bool FWD>
+__global__ void __launch_bounds__(kLevelThreads, 1) k_sweep_levels(DevMesh m, DevState s,
+                                                                  LevelTables lt, int fresh) {
+  if (*s.stop || *s.skip) return;  // converged, or the linear residual dropped below 1e-15
+  extern __shared__ __align__(16) double2 level_smem[];
+  double2* win = level_smem;  // two words a row
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(win + 2 * (lt.ring + 1));
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, r = lane & 3, w = lane >> 2;
+  const int warp = __shfl_sync(FULL, (int)threadIdx.x >> 5, 0);  // uniform in the warp
+  const int nlev = lt.nlev;
+  const int ntile = lt.lev_tile[nlev];
+  const int* load_to = lt.load_to[FWD ? 0 : 1];
+  double2* dqp = reinterpret_cast<double2*>(s.dQ2);  // dQ by position, from 1
+  for (int o = threadIdx.x; o < nlev; o += kLevelThreads) {
+    const int l = FWD ? o : nlev - 1 - o;  // the o-th level to run
+    // the level's tiles, and the loader's lanes for the level after the next
+    level_init(bars + o, (unsigned)(lt.lev_tile[l + 1] - lt.lev_tile[l] + (o + 2 < nlev ? 32 : 0)));
+  }
+  // positions p0 .. p1 - 1 into their places of the ring
+  auto load_window = [&](int p0, int p1, int tid, int nt) {
+    for (int i = 2 * p0 + tid; i < 2 * p1; i += nt) {
+      double2* at = win + 2 * ((i >> 1) % lt.ring) + (i & 1);
+      if (fresh) *at = make_double2(0., 0.);
+      else cp_async16(at, dqp + 2 + i);
+    }
+  };
+  if (threadIdx.x < 2) win[2 * lt.ring + threadIdx.x] = make_double2(0., 0.);
+  const int to1 = load_to[min(1, nlev - 1)];  // the first two levels' rows
+  load_window(FWD ? 0 : to1, FWD ? to1 : m.nn, threadIdx.x, kLevelThreads);
+  cp_async_commit();
+  cp_async_wait<0>();
+  bool timeout = false;
+  if (warp == kLevelWarps) {
+    // ---- the loader ----
+    __syncthreads();
+    int from = to1;
+    for (int o = 2; o < nlev; o++) {
+      const int to = load_to[o];
+      if (o > kLevelsAhead) timeout |= !level_wait(bars + o - 1 - kLevelsAhead, 0);
+      if (FWD) load_window(from, to, lane, 32);
+      else load_window(to, from, lane, 32);
+      from = to;
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(
+                       static_cast<uint32_t>(__cvta_generic_to_shared(bars + o - 2)))
+                   : "memory");
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+  } else {
+    auto tile_at = [&](int k) { return FWD ? k : ntile - 1 - k; };
+    struct Row { int j, block; unsigned ln; int pos; uint4 c; };
+    Row h{}, hn{};
+    double4 a[kRecBlocks];
+    double rhs = 0.;
+    const double4 z4 = make_double4(0., 0., 0., 0.);
+#pragma unroll
+    for (int t = 0; t < kRecBlocks; t++) a[t] = z4;
+    double4 m0 = z4, m1 = z4, m2 = z4, m3 = z4, mr = z4;
+    auto load_row = [&](int k, Row& R) {
+      if (k < ntile) {
+        const LevelSlot* S = lt.slots + 8 * (long)tile_at(k) + w;
+        const int4 q = *reinterpret_cast<const int4*>(S);
+        R.j = q.x;
+        R.block = q.y;
+        R.ln = (unsigned)q.z;
+        R.pos = q.w;
+        R.c = S->cols;
+      }
+    };
+    auto load_tile = [&](int k, const Row& R) {
+      if (k < ntile) {
+        const double* A = s.LHS + 16 * (long)R.block + 4 * r;
+        const int nb = R.ln >> 28;
+#pragma unroll
+        for (int t = 0; t < kRecBlocks; t++) a[t] = t < nb ? ld_d4(A + 16 * t) : z4;
+        rhs = s.RHS[4 * (long)R.j + r];
+        const int j = __shfl_sync(FULL, R.j, 4 * lane);  // row of slot `lane`
+        if (lane < 8) {
+          const double* L = s.LUd + 16 * (long)j;
+          m0 = ld_d4(L);
+          m1 = ld_d4(L + 4);
+          m2 = ld_d4(L + 8);
+          m3 = ld_d4(L + 12);
+          mr = ld_d4(s.LUr + 4 * (long)j);
+        }
+      }
+    };
+    int k = warp;
+    load_row(k, h);
+    load_row(k + kLevelWarps, hn);
+    load_tile(k, h);
+    __syncthreads();
+    for (; k < ntile; k += kLevelWarps) {
+      const int j = __shfl_sync(FULL, h.j, 4 * lane);  // the row lane < 8 solves
+      const int pos = __shfl_sync(FULL, h.pos, 4 * lane);
+      const bool row = j > 0 && lane < 8;
+      const int lev = __shfl_sync(FULL, h.ln & 0xfffffff, 0);
+      const int o = FWD ? lev : nlev - 1 - lev;
+      const double2* d[kRecBlocks] = {
+          win + 2 * (h.c.x & 0xffff), win + 2 * (h.c.x >> 16), win + 2 * (h.c.y & 0xffff),
+          win + 2 * (h.c.y >> 16),    win + 2 * (h.c.z & 0xffff), win + 2 * (h.c.z >> 16),
+          win + 2 * (h.c.w & 0xffff), win + 2 * (h.c.w >> 16)};
+      double2* own = win + 2 * (pos % lt.ring);
+      if (o > 0) timeout |= !level_wait(bars + o - 1, 0);
+      double term[kRecBlocks];
+#pragma unroll
+      for (int t = 0; t < kRecBlocks; t++) {
+        const double2 x01 = d[t][0], x23 = d[t][1];
+        term[t] = (a[t].x * x01.x + a[t].y * x01.y + a[t].z * x23.x + a[t].w * x23.y);
+      }
+      const double2 own01 = own[0], own23 = own[1];
+      // an unused block's term is +0, and acc - 0 is acc, whatever its sign
+      double acc = rhs;
+#pragma unroll
+      for (int t = 0; t < kRecBlocks; t++) acc -= term[t];
+      const double b[4] = {__shfl_sync(FULL, acc, 4 * lane), __shfl_sync(FULL, acc, 4 * lane + 1),
+                           __shfl_sync(FULL, acc, 4 * lane + 2),
+                           __shfl_sync(FULL, acc, 4 * lane + 3)};
+      const double M[16] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w,
+                            m2.x, m2.y, m2.z, m2.w, m3.x, m3.y, m3.z, m3.w};
+      const double rp[4] = {mr.x, mr.y, mr.z, mr.w};
+      double2 x01, x23;
+      if (row) {  // the other lanes' operands would leave the divisions' fast path
+        double X[4];
+        lu_solve4_recip(M, rp, b, X);
+        // dx = X - dQ, dQ + dx (linear_algebra.C:247-262)
+        x01 = make_double2(own01.x + (X[0] - own01.x), own01.y + (X[1] - own01.y));
+        x23 = make_double2(own23.x + (X[2] - own23.x), own23.y + (X[3] - own23.y));
+        own[0] = x01;
+        own[1] = x23;
+      }
+      __syncwarp();
+      if (lane == 0) level_arrive(bars + o);
+      // off the chain: the next tile's loads, this row's result to memory
+      h = hn;
+      asm volatile("" : "+r"(h.j), "+r"(h.block), "+r"(h.ln), "+r"(h.pos)::"memory");
+      asm volatile("" : "+r"(h.c.x), "+r"(h.c.y), "+r"(h.c.z), "+r"(h.c.w)::"memory");
+      load_row(k + 2 * kLevelWarps, hn);
+      load_tile(k + kLevelWarps, h);
+      if (row) {
+        double2* out = reinterpret_cast<double2*>(s.dQ) + 2 * (long)j;
+        out[0] = x01;
+        out[1] = x23;
+        dqp[2 * (long)(pos + 1)] = x01;
+        dqp[2 * (long)(pos + 1) + 1] = x23;
+      }
+    }
+  }
+  if (timeout && lane == 0) atomicOr(s.status, ERR_SWEEP_TIMEOUT);
 }
 
 // Before an ordered sweep: fill its result buffer with the not-ready

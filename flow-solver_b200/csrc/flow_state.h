@@ -120,6 +120,28 @@ struct ChunkTables {
   unsigned* sync;            // dispenser, chunks finished, sweep generation
 };
 
+// FP64 drop-in: the rows of the reference order by dependency level, in tiles
+// of 8 rows (padded at the end of a level), for the ordered sweep
+// k_sweep_levels.  Forward sweeps take the levels ascending, backward ones
+// descending.  A row's position is its place in level order; the sweep's
+// window of dQ is a ring over positions.
+struct LevelSlot {
+  int row;              // 0: an empty slot
+  int block;            // first block of the row
+  unsigned level_nb;    // level, off-diagonal blocks << 28
+  int pos;              // the row's position (from 0)
+  uint4 cols;           // the blocks' columns as 16-bit ring places (the ring's size: none)
+};
+
+struct LevelTables {
+  int nlev;             // 0: the matrix does not take this sweep
+  int ring;             // rows its window of dQ holds
+  const LevelSlot* slots;
+  const int* lev_tile;  // first tile of each level, plus the end
+  const int* load_to[2];  // per direction and level (in its order): positions below (forward)
+                          // or from (backward) it are in the window before the level runs
+};
+
 struct DevState {
   double* Q;
   double* nQ;
@@ -135,6 +157,7 @@ struct DevState {
   double* dt;
   double* LHS;      // nnz * 16
   double* LUd;      // 16 per node: LU factors of the diagonal block
+  double* LUr;      // 4 per node: reciprocals of its pivots (pivot_recip)
   double* xn_bedges;// 3 per bedge (mutated by the k=2 boundary pass)
   double* F;        // 4 per subedge
   double* JL;       // 16 per subedge
