@@ -697,12 +697,8 @@ int launch_linear_solve(flow_ctx* c, const flow_params* p, bool final_rms) {
     }
     if (it < p->subits - 1 || final_rms) {
       Timed t(c, 5);
-      k_lin_residual<<<kRedBlocks, kRedThreads, 0, c->stream>>>(c->m, c->s);
-      rc |= launch_check(c);
-      k_finalize_rms<<<1, kRedThreads, 0, c->stream>>>(c->s, kRedBlocks, c->nn,
-                                                       c->exact_rms);
-      rc |= launch_check(c);
-      k_exact_rms<<<1, 256, 0, c->stream>>>(c->m, c->s);
+      const int nb = std::min(kLinBlocks, grid_blocks(4 * c->nn, kRedThreads));
+      k_lin_residual<<<nb, kRedThreads, 0, c->stream>>>(c->m, c->s, c->exact_rms);
       rc |= launch_check(c);
     }
   }
@@ -1024,7 +1020,7 @@ bool preload_kernels() {
         (const void*)k_sweep_color32<false>, (const void*)k_sweep_ordered32<true>,
         (const void*)k_sweep_ordered32<false>, (const void*)k_prepare_sweep32,
         (const void*)k_fill_sweep_slots, (const void*)k_prepare_sweep,
-        (const void*)k_lin_residual, (const void*)k_finalize_rms, (const void*)k_exact_rms,
+        (const void*)k_lin_residual,
         (const void*)k_finish_step,
         (const void*)k_body_forces,
         (const void*)k_body_forces_sum})
@@ -1794,17 +1790,17 @@ static flow_ctx* create_impl(flow_arena* arena, const flow_grid_view* g, const f
   s.counter = c->buf.alloc<unsigned>(4);
   s.status = c->buf.alloc<int>(1);
   s.skip = c->buf.alloc<int>(1);
-  s.exact = c->buf.alloc<int>(1);
   s.stop = c->buf.alloc<int>(1);
   s.steps_done = c->buf.alloc<int>(1);
   s.citer = c->buf.alloc<int>(1);
-  // the partial sums of the step's reductions, then k_finish_step's block count
-  s.partial = c->buf.alloc<double>(2 * kRedBlocks + 2);
+  // the partial sums of the step's reductions and k_finish_step's block count,
+  // then those of k_lin_residual
+  s.partial = c->buf.alloc<double>(kLinPartial + kLinBlocks + 2);
   s.scalars = c->buf.alloc<double>(8);
   if (!s.Q || !s.nQ || !s.pQ || !s.dQ || !s.dQ2 || !s.R || !s.RHS || !s.grad || !s.phi || !s.hess5 ||
       !s.pv || !s.dt || !s.LHS || !s.LUd || !s.xn_bedges || !s.F || !s.JL || !s.JR || !s.Fb ||
       !s.Jb || !s.bforce || !s.done || !s.counter || !s.status || !s.skip || !s.partial ||
-      !s.scalars || !s.stop || !s.steps_done || !s.citer || !s.exact)
+      !s.scalars || !s.stop || !s.steps_done || !s.citer)
     return fail(c, carve_error(c), "device state allocation failed");
   bool zero_ok = true;
   auto zero = [&](void* ptr, size_t bytes) {
@@ -1826,12 +1822,11 @@ static flow_ctx* create_impl(flow_arena* arena, const flow_grid_view* g, const f
   zero(s.done, (size_t)(nn + 1) * 4);
   zero(s.status, 4);
   zero(s.skip, 4);
-  zero(s.exact, 4);
   zero(s.stop, 4);
   zero(s.steps_done, 4);
   zero(s.citer, 4);
   zero(s.scalars, 64);
-  zero(s.partial, (2 * kRedBlocks + 2) * 8);
+  zero(s.partial, (kLinPartial + kLinBlocks + 2) * 8);
   if (!zero_ok) return fail(c, FLOW_ERR_CUDA, "clearing the device state failed");
   std::vector<double> xnb((size_t)(nbe + 1) * 3, 0.);
   std::copy(g->xn_bedges, g->xn_bedges + xnb.size(), xnb.begin());
@@ -2817,85 +2812,69 @@ double flow_last_device_ms(flow_ctx* c) { return c ? c->last_ms : 0.; }
 // start-up (a cudaMalloc behind the arena's back fails once it holds the
 // GPU, or fragments it), and time-step loops that must not take the implicit
 // device-wide synchronisation that cudaMalloc and cudaFree can cause.  The
-// kernels below are the per-sweep residual of flow_linear_solve
-// (k_lin_residual + k_finalize_rms) with their scratch moved into one
-// file-scope __device__ array: the squared residual of each row, the block
-// partial sums, the RMS and an error word.  The partial sums follow
-// k_lin_residual's order, so the RMS is the one flow_linear_solve returns for
-// the same matrix, right-hand side and dQ.
+// kernel below is the per-sweep residual of flow_linear_solve
+// (k_lin_residual) with its scratch moved into one file-scope __device__
+// array: the block partial sums, the RMS, an error word and the block count.
+// The partial sums follow k_lin_residual's order, so the RMS is the one
+// flow_linear_solve returns for the same matrix, right-hand side and dQ.
+// FLOW_NOALLOC_MAX_ROWS stays the interface's limit.
 // ===========================================================================
 namespace flow {
 namespace noalloc {
-constexpr long kRowOff = 0;                                 // [1, nn]: |r_j|^2
-constexpr long kPartOff = (long)FLOW_NOALLOC_MAX_ROWS + 1;  // kRedBlocks block sums
-constexpr long kOutOff = kPartOff + kRedBlocks;             // RMS, then the error word
-constexpr long kWords = ((kOutOff + 2 + 31) / 32) * 32;
+constexpr long kPartOff = 0;             // kLinBlocks block sums
+constexpr long kOutOff = kLinBlocks;     // RMS, then the error word and the block count
+constexpr long kWords = ((kOutOff + 3 + 31) / 32) * 32;
 constexpr int kMaxDevices = 64;
 constexpr unsigned long long kBadRowPtr = 1ull, kBadColumn = 2ull;
 }  // namespace noalloc
 }  // namespace flow
 
-// The scratch of flow_linear_residual_noalloc: about 2 MB per device, shared
-// by every call on that device.
+// The scratch of flow_linear_residual_noalloc, shared by every call on its
+// device.
 static __device__ __align__(256) double g_noalloc_scratch[flow::noalloc::kWords];
 
 namespace flow {
 namespace noalloc {
 
-// Squared residual of every row; the residual itself is formed exactly as in
-// k_lin_residual.  Row pointers and columns outside the system are reported
-// in the error word and never dereferenced.
+// The RMS in one launch, formed as k_lin_residual forms it.  Row pointers and
+// columns outside the system are reported in the error word and never
+// dereferenced.  ALIGNED: lhs and x on 32-byte boundaries (block rows and rows
+// of x in one access each); callers' pointers need only be 8-byte aligned.
+template <bool ALIGNED>
 __global__ void __launch_bounds__(kRedThreads)
-    k_rows(const int* ia, const int* ja, const double* lhs, const double* rhs, const double* x,
-           int nn, long nnz, double* scratch) {
+    k_rms(const int* ia, const int* ja, const double* lhs, const double* rhs, const double* x,
+          int nn, long nnz, double* scratch) {
+  __shared__ double sh[kRedThreads];
+  __shared__ int is_last;
   unsigned long long* err = reinterpret_cast<unsigned long long*>(scratch + kOutOff + 1);
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x + 1; j <= nn;
-       j += gridDim.x * blockDim.x) {
-    double r[4] = {rhs[4 * (long)j], rhs[4 * (long)j + 1], rhs[4 * (long)j + 2],
-                   rhs[4 * (long)j + 3]};
-    const int k0 = ia[j], k1 = ia[j + 1];
-    if (k0 < 0 || k1 < k0 || (long)k1 > nnz) {
-      atomicOr(err, kBadRowPtr);
-      scratch[kRowOff + j] = 0.;
-      continue;
-    }
-    for (int k = k0; k < k1; k++) {
-      const int c = ja[k];
-      if (c < 1 || c > nn) {
-        atomicOr(err, kBadColumn);
-        continue;
-      }
-      const double d[4] = {x[4 * (long)c], x[4 * (long)c + 1], x[4 * (long)c + 2],
-                           x[4 * (long)c + 3]};
-      const double* A = lhs + 16 * (long)k;
-#pragma unroll
-      for (int q = 0; q < 4; q++) r[q] -= row_dot(A, q, d);
-    }
-    scratch[kRowOff + j] = (r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3]);
-  }
-}
-
-// Block partial sums over the same rows, in the same order, as k_lin_residual.
-__global__ void __launch_bounds__(kRedThreads) k_partials(int nn, double* scratch) {
-  __shared__ double sh[kRedThreads];
-  double acc = 0.;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x + 1; j <= nn;
-       j += gridDim.x * blockDim.x)
-    acc += scratch[kRowOff + j];
-  double tot = block_sum(acc, sh);
-  if (threadIdx.x == 0) scratch[kPartOff + blockIdx.x] = tot;
-}
-
-// The RMS from the partials, as k_finalize_rms forms it.
-__global__ void __launch_bounds__(kRedThreads) k_rms(int nn, double* scratch) {
-  __shared__ double sh[kRedThreads];
-  double v = 0.;
-  for (int i = threadIdx.x; i < kRedBlocks; i += blockDim.x) v += scratch[kPartOff + i];
-  double tot = block_sum(v, sh);
+  unsigned* done = reinterpret_cast<unsigned*>(scratch + kOutOff + 2);
+  const double tot = block_residual2<ALIGNED>(
+      ia, ja, lhs, rhs, x, nn, sh,
+      [&](int k0, int k1) {
+        const bool ok = k0 >= 0 && k1 >= k0 && (long)k1 <= nnz;
+        if (!ok) atomicOr(err, kBadRowPtr);
+        return ok;
+      },
+      [&](int c) {
+        const bool ok = c >= 1 && c <= nn;
+        if (!ok) atomicOr(err, kBadColumn);
+        return ok;
+      });
   if (threadIdx.x == 0) {
-    double rms = tot / (1. * nn);
-    rms = sqrt(rms);
-    scratch[kOutOff] = rms;
+    scratch[kPartOff + blockIdx.x] = tot;
+    __threadfence();  // the partial is visible before the count says so
+    is_last = atomicAdd(done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!is_last) return;
+  __threadfence();
+  double v = 0.;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += kRedThreads)
+    v += __ldcg(scratch + kPartOff + i);
+  const double sum = block_sum(v, sh);
+  if (threadIdx.x == 0) {
+    double rms = sum / (1. * nn);
+    scratch[kOutOff] = sqrt(rms);
   }
 }
 
@@ -2971,14 +2950,15 @@ extern "C" int flow_linear_residual_noalloc(const int* ia, const int* ja, const 
   double* scratch = scratch_for(dev, &rc);
   if (!scratch) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // The error word must start at zero; every other word this call reads, it
-  // writes first.
-  e = cudaMemsetAsync(scratch + kOutOff + 1, 0, sizeof(double), st);
+  // The error word and the block count must start at zero; every other word
+  // this call reads, it writes first.
+  e = cudaMemsetAsync(scratch + kOutOff + 1, 0, 2 * sizeof(double), st);
   if (e == cudaSuccess) {
-    k_rows<<<flow::kRedBlocks, flow::kRedThreads, 0, st>>>(ia, ja, lhs, rhs, x, nn, nnz,
-                                                           scratch);
-    k_partials<<<flow::kRedBlocks, flow::kRedThreads, 0, st>>>(nn, scratch);
-    k_rms<<<1, flow::kRedThreads, 0, st>>>(nn, scratch);
+    const int nb = std::min(flow::kLinBlocks, grid_blocks(4 * nn, flow::kRedThreads));
+    if (((uintptr_t)lhs | (uintptr_t)x) % 32 == 0)
+      k_rms<true><<<nb, flow::kRedThreads, 0, st>>>(ia, ja, lhs, rhs, x, nn, nnz, scratch);
+    else
+      k_rms<false><<<nb, flow::kRedThreads, 0, st>>>(ia, ja, lhs, rhs, x, nn, nnz, scratch);
     e = cudaGetLastError();
   }
   double out[2] = {0., 0.};

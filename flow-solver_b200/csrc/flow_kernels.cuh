@@ -2311,86 +2311,141 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
   return out;
 }
 
-// b - Ax of every row (linear_algebra.C:348-387), squared, partial sums.
-__global__ void __launch_bounds__(kRedThreads) k_lin_residual(DevMesh m, DevState s) {
-  if (*s.stop) return;  // the run has converged
-  __shared__ double sh[kRedThreads];
-  double acc = 0.;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x + 1; j <= m.nn;
-       j += gridDim.x * blockDim.x) {
-    double r[4];
-    const double4 rh = reinterpret_cast<const double4*>(s.RHS)[j];
-    r[0] = rh.x; r[1] = rh.y; r[2] = rh.z; r[3] = rh.w;
-    for (int k = m.ia[j]; k < m.ia[j + 1]; k++) {
-      const double4 d4 = reinterpret_cast<const double4*>(s.dQ)[m.ja[k]];
-      const double d[4] = {d4.x, d4.y, d4.z, d4.w};
-      const double* A = s.LHS + 16 * (long)k;
-#pragma unroll
-      for (int q = 0; q < 4; q++) r[q] -= row_dot(A, q, d);
-    }
-    acc += (r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3]);
-  }
-  double tot = block_sum(acc, sh);
-  if (threadIdx.x == 0) s.partial[blockIdx.x] = tot;
+// A double4 of data the kernel does not write, in one 32-byte access (ALIGNED:
+// p on a 32-byte boundary) or as four values.
+template <bool ALIGNED>
+__device__ __forceinline__ double4 ldg_d4(const double* p) {
+  double4 v;
+  if (ALIGNED)
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+        : "l"(p));
+  else
+    v = make_double4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+  return v;
 }
 
-// Sum the partials in a fixed order; slot 0 = RMS (sets skip below 1e-15).
-// The tree sum differs from the reference's row-order sum by at most
+// |b - Ax|^2 of the rows by quads of lanes, lane q owning component q: row j's
+// components as the reference forms them (linear_algebra.C:348-387), squared
+// and added in component order (in every lane of the quad).  ok(k0, k1) checks
+// the row's block range and ok_col(c) a column before they are used.
+template <bool ALIGNED, class Rows, class Col>
+__device__ __forceinline__ double row_residual2(const int* ia, const int* ja, const double* lhs,
+                                                const double* rhs, const double* x, int j, int q,
+                                                unsigned qmask, int qbase, Rows&& ok,
+                                                Col&& ok_col) {
+  double r = __ldg(rhs + 4 * (long)j + q);
+  const int k0 = __ldg(ia + j), k1 = __ldg(ia + j + 1);
+  if (!ok(k0, k1)) return 0.;  // the whole quad
+  // four blocks at a time, their loads issued together
+  for (int k = k0; k < k1; k += 4) {
+    int c[4];
+    double4 a[4], d[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int ki = min(k + i, k1 - 1);
+      c[i] = __ldg(ja + ki);
+      a[i] = ldg_d4<ALIGNED>(lhs + 16 * (long)ki + 4 * q);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      if (!ok_col(c[i])) c[i] = 0;  // left out below; row 1 of x stands in
+      d[i] = ldg_d4<ALIGNED>(x + 4 * (long)max(c[i], 1));
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      if (k + i < k1 && c[i] > 0)
+        r -= (a[i].x * d[i].x + a[i].y * d[i].y + a[i].z * d[i].z + a[i].w * d[i].w);
+  }
+  const double r2 = r * r;
+  const double s0 = __shfl_sync(qmask, r2, qbase), s1 = __shfl_sync(qmask, r2, qbase + 1);
+  const double s2 = __shfl_sync(qmask, r2, qbase + 2), s3 = __shfl_sync(qmask, r2, qbase + 3);
+  return s0 + s1 + s2 + s3;
+}
+
+// The sum of row_residual2 over the block's rows, by thread 0.
+template <bool ALIGNED, class Rows, class Col>
+__device__ __forceinline__ double block_residual2(const int* ia, const int* ja, const double* lhs,
+                                                  const double* rhs, const double* x, int nn,
+                                                  double* sh, Rows&& ok, Col&& ok_col) {
+  const int q = threadIdx.x & 3, qbase = threadIdx.x & 31 & ~3;
+  const unsigned qmask = 0xFu << qbase;
+  double acc = 0.;
+  for (int j = (blockIdx.x * blockDim.x + threadIdx.x) / 4 + 1; j <= nn;
+       j += gridDim.x * blockDim.x / 4) {
+    const double v = row_residual2<ALIGNED>(ia, ja, lhs, rhs, x, j, q, qmask, qbase, ok, ok_col);
+    if (q == 0) acc += v;
+  }
+  return block_sum(acc, sh);
+}
+
+// b - Ax RMS of the linear solve, its partial sums by block; the last block to
+// finish sums those in a fixed order and sets the RMS and the skip flag below
+// 1e-15.  The tree sum differs from the reference's row-order sum by at most
 // (nn-1) u of the sum (u = 2^-53, every term is positive), so the RMS by at
 // most about half that: when the RMS lies that close to the 1e-15 test of
-// linear_algebra.C:387, k_exact_rms settles the test in the reference's order.
-__global__ void k_finalize_rms(DevState s, int nparts, int nn, int always_exact) {
+// linear_algebra.C:387 (or always, always_exact), that block sums the rows
+// again in the reference's order, 256 rows' squared residuals at a time added
+// by thread 0, and the test takes that value.
+//
+// Bound by HBM (the matrix once).  Four lanes a row read whole 32-byte block
+// rows, four blocks' loads in flight; 181k rows 116 -> 45 us (3.7 TB/s of
+// compulsory bytes), 65,536 49 -> 23, and below 10k rows, where three launches
+// were the time, 30 -> 11.
+constexpr int kLinBlocks = 1184;  // 8 a SM; fixed so that the sum is deterministic
+constexpr int kLinPartial = 2 * kRedBlocks + 2;  // first of them in DevState::partial, then a count
+__global__ void __launch_bounds__(kRedThreads) k_lin_residual(DevMesh m, DevState s,
+                                                              int always_exact) {
   if (*s.stop) return;  // the run has converged
   __shared__ double sh[kRedThreads];
+  __shared__ int is_last;
+  auto any = [](auto...) { return true; };
+  const double tot =
+      block_residual2<true>(m.ia, m.ja, s.LHS, s.RHS, s.dQ, m.nn, sh, any, any);
+  double* part = s.partial + kLinPartial;
+  unsigned* done = reinterpret_cast<unsigned*>(part + kLinBlocks);
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = tot;
+    __threadfence();  // the partial is visible before the count says so
+    is_last = atomicAdd(done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!is_last) return;
+  __threadfence();
   double v = 0.;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) v += s.partial[i];
-  double tot = block_sum(v, sh);
-  if (threadIdx.x == 0) {
-    double rms = tot / (1. * nn);
-    rms = sqrt(rms);
-    s.scalars[0] = rms;
-    if (rms < 1.0E-15) *s.skip = 1;
-    if (always_exact || fabs(rms - 1.0E-15) <= 1.0E-15 * ((nn + 16.) * 2.3e-16)) *s.exact = 1;
-  }
-}
-
-// The b - Ax RMS in the reference's order (linear_algebra.C:348-387), run only
-// when k_finalize_rms found the tree RMS within its error bound of 1e-15: the
-// CTA forms 256 rows' squared residuals at a time, thread 0 adds them in row
-// order.  It sets the RMS and the skip flag as the reference's test decides.
-__global__ void __launch_bounds__(256) k_exact_rms(DevMesh m, DevState s) {
-  if (*s.stop || !*s.exact) return;
-  __shared__ double term[256];
-  double acc = 0.;
-  for (int j0 = 1; j0 <= m.nn; j0 += 256) {
-    const int j = j0 + threadIdx.x;
-    if (j <= m.nn) {
-      double r[4];
-      const double4 rh = reinterpret_cast<const double4*>(s.RHS)[j];
-      r[0] = rh.x; r[1] = rh.y; r[2] = rh.z; r[3] = rh.w;
-      for (int k = m.ia[j]; k < m.ia[j + 1]; k++) {
-        const double4 d4 = reinterpret_cast<const double4*>(s.dQ)[m.ja[k]];
-        const double d[4] = {d4.x, d4.y, d4.z, d4.w};
-        const double* A = s.LHS + 16 * (long)k;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += kRedThreads) v += __ldcg(part + i);
+  double sum = block_sum(v, sh);
+  double rms = sqrt(sum / (1. * m.nn));
+  if (always_exact || fabs(rms - 1.0E-15) <= 1.0E-15 * ((m.nn + 16.) * 2.3e-16)) {
+    sum = 0.;
+    for (int j0 = 1; j0 <= m.nn; j0 += kRedThreads) {
+      const int j = j0 + threadIdx.x;
+      if (j <= m.nn) {
+        const double4 rh = reinterpret_cast<const double4*>(s.RHS)[j];
+        double r[4] = {rh.x, rh.y, rh.z, rh.w};
+        for (int k = m.ia[j]; k < m.ia[j + 1]; k++) {
+          const double4 d4 = reinterpret_cast<const double4*>(s.dQ)[m.ja[k]];
+          const double d[4] = {d4.x, d4.y, d4.z, d4.w};
 #pragma unroll
-        for (int q = 0; q < 4; q++) r[q] -= row_dot(A, q, d);
+          for (int q = 0; q < 4; q++) r[q] -= row_dot(s.LHS + 16 * (long)k, q, d);
+        }
+        sh[threadIdx.x] = (r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3]);
       }
-      term[threadIdx.x] = (r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3]);
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        const int cnt = min(kRedThreads, m.nn - j0 + 1);
+        for (int t = 0; t < cnt; t++) sum += sh[t];
+      }
+      __syncthreads();
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const int cnt = min(256, m.nn - j0 + 1);
-      for (int t = 0; t < cnt; t++) acc += term[t];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    double rms = acc;
+    rms = sum;
     rms /= (1. * m.nn);
     rms = sqrt(rms);
+  }
+  if (threadIdx.x == 0) {
     s.scalars[0] = rms;
-    *s.skip = rms < 1.0E-15 ? 1 : 0;
-    *s.exact = 0;
+    if (rms < 1.0E-15) *s.skip = 1;
+    *done = 0u;
   }
 }
 

@@ -598,15 +598,15 @@ const char *flow_server_last_error(void);
  * for it and stores the RMS in the host double *rms.  A row pointer or
  * column outside the system is reported as FLOW_ERR_ARG.
  *
- * Scratch: one file-scope __device__ array per device (about 2 MB), sized
- * for FLOW_NOALLOC_MAX_ROWS rows; a larger nn is rejected with FLOW_ERR_ARG
- * and a message in flow_last_error().  The first call on each device does a
+ * Scratch: one file-scope __device__ array per device (about 10 KB); an nn
+ * above FLOW_NOALLOC_MAX_ROWS rows is rejected with FLOW_ERR_ARG and a
+ * message in flow_last_error().  The first call on each device does a
  * one-time set-up (its look-up of the array's device address also loads
  * this library's device code on that device): make that first call before
  * any stream capture starts.  Later calls look the address up again, which
  * allocates nothing and follows a module reloaded after cudaDeviceReset.
  * Every call on a device shares the array, which
- * keeps the last call's contents; each call clears the one word that must
+ * keeps the last call's contents; each call clears the words that must
  * start at zero.  Calls whose GPU work overlaps (several host threads on
  * different streams) race on the array and return wrong results: serialise
  * them. */
