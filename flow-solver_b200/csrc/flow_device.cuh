@@ -314,36 +314,68 @@ __device__ __forceinline__ double venkat_fold(double ph, double qrec, double q0,
   return ph <= b ? ph : b;
 }
 
-// venkat_fold without a division of a zero or by a zero: a point the fold
-// discards (qrec == q0, or a NaN difference) and a point whose bound is the
-// node's own value (qmax == q0 going up, qmin == q0 going down: a zero
-// dividend) divide 1 by 1 instead.  The first folds in 1 as before; the
-// second folds in +0, the bits the reference's quotients give there
-// (0/d = +-0, then (+0 + +-0) / (+0 +- 0 + 2) = +0).  Every other point
-// divides the same operands, so phi has the same bits.  Where the state is
-// uniform (the free stream of the first steps) most points are of the two
-// kinds, and a division of or by zero leaves the fast path of the division.
-__device__ __forceinline__ double venkat_fold_nz(double ph, double qrec, double q0, double qmin,
-                                                 double qmax) {
-  const double d = qrec - q0;
-  const bool up = d > 0., down = d < 0.;
-  const bool used = up || down;
-  const double num = up ? qmax - q0 : qmin - q0;
-  const bool flat = num == 0.;
-  const bool div = used && !flat;
-  double t = (div ? num : 1.0) / (div ? d : 1.0);
-  t = (t * t + 2. * t) / (t * t + t + 2.);
-  const double b = used ? (flat ? 0.0 : t) : 1.0;
-  return ph <= b ? ph : b;
-}
+// The minimum of venkat_fold over a node's face points without two divisions a
+// point.  With d = qrec - q0, a point's bound is phi(t), t = (qmax - q0) / d
+// going up and (qmin - q0) / d going down: on either side the quotients are
+// ordered as |d| (a division is monotone, rounded or not), and phi rises up to
+// 1 at t = 2, so the side's smallest bound is that of its largest |d|, and two
+// divisions a side give it.  In rounded arithmetic phi(t) carries a relative
+// error below 6 u (u = 2^-53) while t phi'/phi >= 1/4 on (0, 2]: a point whose
+// t is larger by 48 u or more cannot have the smaller computed bound, and
+// beyond t = 2 (1 + 24 u) the computed bound is at least 1, which the fold
+// ignores.  So the result is the fold's, bit for bit, unless another |d| of
+// the side is as large to a relative 2^-22 (equal ones too: the scan compares
+// d in FP32), or a quotient's square may overflow or a |d| underflow in FP32
+// (tiny), or a bound is not finite; then the caller folds the points one by
+// one.  Points with d zero or NaN fold in 1, as in venkat_fold.
+struct LimiterScan {
+  double up = 0., down = 0.;     // the d of each side with the largest magnitude (0: none)
+  float up1 = 0.f, up2 = 0.f;    // its magnitude and the second largest, in FP32
+  float down1 = 0.f, down2 = 0.f;
+  bool tiny = false;
 
-// The limiter fold of a node kernel: 0 venkat_fold, 1 or 2 venkat_fold_nz.
-template <int LIM>
-__device__ __forceinline__ double venkat_fold_lim(double ph, double qrec, double q0, double qmin,
-                                                  double qmax) {
-  if (LIM >= 1) return venkat_fold_nz(ph, qrec, q0, qmin, qmax);
-  return venkat_fold(ph, qrec, q0, qmin, qmax);
-}
+  __device__ __forceinline__ void add(double d) {
+    const float f = __double2float_rn(d);
+    // a max or min with a NaN is the other operand
+    up = f > up1 ? d : up;
+    up2 = fmaxf(up2, fminf(up1, f));
+    up1 = fmaxf(up1, f);
+    down = -f > down1 ? d : down;
+    down2 = fmaxf(down2, fminf(down1, -f));
+    down1 = fmaxf(down1, -f);
+    tiny = tiny || (fabsf(f) < 1e-30f && d != 0.);
+  }
+  // another scan's points
+  __device__ __forceinline__ void merge(double oup, float oup1, float oup2, double odown,
+                                        float odown1, float odown2, bool otiny) {
+    up = oup1 > up1 ? oup : up;
+    up2 = fmaxf(fmaxf(up2, oup2), fminf(up1, oup1));
+    up1 = fmaxf(up1, oup1);
+    down = odown1 > down1 ? odown : down;
+    down2 = fmaxf(fmaxf(down2, odown2), fminf(down1, odown1));
+    down1 = fmaxf(down1, odown1);
+    tiny = tiny || otiny;
+  }
+  // the scan's result stands for bounds a_up = qmax - q0, a_down = qmin - q0
+  __device__ __forceinline__ bool settled(double a_up, double a_down) const {
+    constexpr float kNear = 1.f - 0x1p-22f;
+    return !tiny && (up2 == 0.f || up2 < kNear * up1) && (down2 == 0.f || down2 < kNear * down1) &&
+           a_up < 1e120 && a_down > -1e120;
+  }
+  // a zero dividend's bound is +0 (0 / d = +-0, then (+0 + +-0) / (+0 +- 0 + 2) = +0)
+  // and is not divided: a division of a zero leaves the division's fast path
+  __device__ __forceinline__ static double bound(double a, double d) {
+    const bool div = d != 0. && a != 0.;
+    double t = (div ? a : 1.0) / (div ? d : 1.0);
+    t = (t * t + 2. * t) / (t * t + t + 2.);
+    return d != 0. ? (a != 0. ? t : 0.0) : 1.0;
+  }
+  __device__ __forceinline__ double phi(double a_up, double a_down) const {
+    const double b0 = bound(a_up, up), b1 = bound(a_down, down);
+    const double ph = 1.0 <= b0 ? 1.0 : b0;
+    return ph <= b1 ? ph : b1;
+  }
+};
 
 // linear_algebra.C:571-596 lu() on a 4x4 row-major block, in place.
 __device__ __forceinline__ void lu4(double* A) {

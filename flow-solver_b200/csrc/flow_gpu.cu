@@ -191,7 +191,7 @@ struct flow_ctx {
   // precision form (flow_set_precision): 0 FP64 reference order, 1 FP32
   // blocks with multicolour sweeps; tables built on first use
   int precision = 0;
-  int var[2] = {0, 0};  // kernel variants: k_node_prepare4, k_subedge_flux (autotuner)
+  int var[2] = {0, 0};  // kernel variants: the node kernel (default_node_variant), k_subedge_flux
   int sched_sweeps = 0, sched_until = 0;  // sweep schedule (flow_set_sweep_schedule)
   MixedTables mt{};
   bool mt_ordered = false;  // tables in reference row order (modes 2, 3) or colour order (mode 1)
@@ -370,31 +370,51 @@ void harvest(flow_ctx* c) {
   c->pending.clear();
 }
 
-// Kernel variants the autotuner chooses between: minimum resident blocks per
-// SM in __launch_bounds__ (which caps the registers per thread).
-// k_node_prepare4: variant 0, 1, 2 -> 0 (compiler's choice), 10, 12 blocks.
-// k_subedge_flux:  variant 0, 1, 2 -> 4, 5, 3 blocks.
+// Kernel variants the autotuner chooses between.  k_subedge_flux: variant 0, 1,
+// 2 -> at least 4, 5, 3 resident blocks per SM (__launch_bounds__, which caps
+// the registers per thread).  The node kernel: k_node_prepare4 in the forms of
+// node_kernel, variant 3 = k_node_stage (gathers staged in shared memory) where
+// its shared memory fits the mesh, variant 7 = k_node_prepare16 (each node's
+// chains split over 16 lanes).
 constexpr int kVariants = 3;
-// k_node_prepare4 has five more: variant 3 = k_node_stage (gathers staged in
-// shared memory), where its shared memory fits the mesh; variant 4 =
-// k_node_prepare16 (each node's chains split over 16 lanes); variants 5, 6
-// and 7 = variants 0, 1 and 4 with the limiter fold that divides no zero
-// and by no zero (venkat_fold_nz), variant 5 with the wave-speed face terms
-// in the limiter's face loop too (LIM = 2; variants 6 and 7 LIM = 1).
 constexpr int kNodeVariants = 8;
 constexpr int kLevelSmemMax = 227 * 1024;  // k_sweep_levels
 constexpr size_t kStageSmemMax = 110 * 1024;  // two CTAs per SM at most
-template <class F>
-void launch_variant(int v, F&& f) {
-  if (v == 1) f(std::integral_constant<int, 10>());
-  else if (v == 2) f(std::integral_constant<int, 12>());
-  else f(std::integral_constant<int, 0>());
+using NodeKernel = void (*)(DevMesh, DevState, StepArgs);
+struct NodeForm {
+  NodeKernel kernel;
+  int lanes;  // of a node
+};
+template <int ORDER, int MINB, bool MERGED, int NV>
+constexpr NodeForm node_form() {
+  return {k_node_prepare4<ORDER, MINB, MERGED, NV>, 4 / NV};
 }
-// node variants 5 and 6: (MINB, LIM) = (0, 2) and (10, 1)
-template <class F>
-void launch_lim_variant(int v, F&& f) {
-  if (v == 6) f(std::integral_constant<int, 10>(), std::integral_constant<int, 1>());
-  else f(std::integral_constant<int, 0>(), std::integral_constant<int, 2>());
+NodeForm node_kernel(bool k1, int v) {
+  if (v == 7) return {k1 ? k_node_prepare16<1> : k_node_prepare16<3>, 16};
+  switch (v) {
+    case 1: return k1 ? node_form<1, 8, false, 1>() : node_form<3, 7, false, 1>();
+    case 2: return k1 ? node_form<1, 6, false, 2>() : node_form<3, 4, true, 2>();
+    case 4: return k1 ? node_form<1, 5, true, 1>() : node_form<3, 5, true, 1>();
+    case 5: return k1 ? node_form<1, 4, true, 2>() : node_form<3, 4, false, 2>();
+    case 6: return k1 ? node_form<1, 10, false, 1>() : node_form<3, 8, false, 1>();
+    default: return k1 ? node_form<1, 6, true, 1>() : node_form<3, 6, false, 1>();
+  }
+}
+// The node variant of a context that is not autotuned: the form with the
+// shortest chains whose blocks are all resident at once (resident blocks x
+// nodes a block), as a second wave costs a whole pass of a block; where none
+// is, the form that is fastest over several waves.  us, k=2: 2,116 nodes 19
+// with 16 lanes, 23 with variant 0; 25,600 43 / 44 / 50 with 0 / 1 / 2; 65,536
+// (two waves of variant 1) 84 / 77 / 81; 181k 187 / 187 / 170.  k=1: 25,600
+// 21 / 23 / 25, 40,804 35 / 35 / 28, 65,536 47 / 39 / 43, 181k 94 / 84 / 78.
+int default_node_variant(int order, int nn, int nsm) {
+  if (order == 3 && nn < 5000) return 7;
+  const int w0 = 6 * 32 * nsm, w1 = (order == 3 ? 7 : 8) * 32 * nsm,
+            w2 = (order == 3 ? 4 : 6) * 64 * nsm;
+  if (nn <= w0) return 0;
+  if (nn <= w1) return 1;
+  if (nn <= w2) return 2;
+  return nn <= 2 * w1 ? 1 : 2;
 }
 template <class F>
 void launch_flux_variant(int v, F&& f) {
@@ -409,21 +429,9 @@ int launch_node_prepare(flow_ctx* c, const StepArgs& a) {
     return FLOW_ERR_ARG;
   }
   Timed tm(c, 0);
-  int nb = grid_blocks(4 * c->nn, 128);
   // the LSQ gradient (k=1, or the second-order start-up steps of k=2) is
   // the k=1 kernel's work
   const bool k1 = c->order == 1 || a.do_grad;
-  if (c->var[0] == 4 || c->var[0] == 7) {
-    const int nb16 = grid_blocks(16 * c->nn, 128);
-    if (c->var[0] == 7) {
-      if (k1) k_node_prepare16<1, 1><<<nb16, 128, 0, c->stream>>>(c->m, c->s, a);
-      else k_node_prepare16<3, 1><<<nb16, 128, 0, c->stream>>>(c->m, c->s, a);
-    } else {
-      if (k1) k_node_prepare16<1><<<nb16, 128, 0, c->stream>>>(c->m, c->s, a);
-      else k_node_prepare16<3><<<nb16, 128, 0, c->stream>>>(c->m, c->s, a);
-    }
-    return launch_check(c);
-  }
   if (c->var[0] == 3 && c->stage_ok[k1 ? 0 : 1]) {
     const int tiles = grid_blocks(c->nn, kStageNodes);
     if (k1)
@@ -434,25 +442,8 @@ int launch_node_prepare(flow_ctx* c, const StepArgs& a) {
           c->m, c->s, a, c->stage_caps);
     return launch_check(c);
   }
-  if (c->var[0] >= 5) {
-    if (k1)
-      launch_lim_variant(c->var[0], [&](auto W, auto L) {
-        k_node_prepare4<1, W.value, L.value><<<nb, 128, 0, c->stream>>>(c->m, c->s, a);
-      });
-    else
-      launch_lim_variant(c->var[0], [&](auto W, auto L) {
-        k_node_prepare4<3, W.value, L.value><<<nb, 128, 0, c->stream>>>(c->m, c->s, a);
-      });
-    return launch_check(c);
-  }
-  if (k1)
-    launch_variant(c->var[0], [&](auto V) {
-      k_node_prepare4<1, V.value><<<nb, 128, 0, c->stream>>>(c->m, c->s, a);
-    });
-  else
-    launch_variant(c->var[0], [&](auto V) {
-      k_node_prepare4<3, V.value><<<nb, 128, 0, c->stream>>>(c->m, c->s, a);
-    });
+  const NodeForm f = node_kernel(k1, c->var[0]);
+  f.kernel<<<grid_blocks(f.lanes * c->nn, 128), 128, 0, c->stream>>>(c->m, c->s, a);
   return launch_check(c);
 }
 
@@ -989,19 +980,12 @@ bool preload_kernels() {
   bool ok = true;
   for (const void* f :
        {(const void*)k_step_args, (const void*)k_begin_step,
-        (const void*)k_node_prepare4<1, 0>, (const void*)k_node_prepare4<1, 10>,
-        (const void*)k_node_prepare4<1, 12>, (const void*)k_node_prepare4<3, 0>,
-        (const void*)k_node_prepare4<3, 10>, (const void*)k_node_prepare4<3, 12>,
-        (const void*)k_node_prepare4<1, 0, 2>, (const void*)k_node_prepare4<1, 10, 1>,
-        (const void*)k_node_prepare4<3, 0, 2>, (const void*)k_node_prepare4<3, 10, 1>,
         (const void*)k_assemble4<true, 0>, (const void*)k_assemble4<false, 0>,
         (const void*)k_assemble4<true, 1>, (const void*)k_assemble4<false, 1>,
         (const void*)k_assemble4<true, 2>, (const void*)k_assemble4<false, 2>,
         (const void*)k_assemble4<true, 1, true>, (const void*)k_assemble4<true, 2, true>,
         (const void*)k_boundary_add4<true>, (const void*)k_boundary_add4<false>,
         (const void*)k_node_stage<1>, (const void*)k_node_stage<3>,
-        (const void*)k_node_prepare16<1>, (const void*)k_node_prepare16<3>,
-        (const void*)k_node_prepare16<1, 1>, (const void*)k_node_prepare16<3, 1>,
         (const void*)k_faces_assemble<0, 1>, (const void*)k_faces_assemble<1, 1>,
         (const void*)k_faces_assemble<0, 2>, (const void*)k_faces_assemble<1, 2>,
         (const void*)k_diag_lu,
@@ -1025,6 +1009,9 @@ bool preload_kernels() {
         (const void*)k_body_forces,
         (const void*)k_body_forces_sum})
     ok = ok && cudaFuncGetAttributes(&fa, f) == cudaSuccess;
+  for (int v = 0; v < kNodeVariants; v++)
+    for (bool k1 : {false, true})
+      ok = ok && cudaFuncGetAttributes(&fa, (const void*)node_kernel(k1, v).kernel) == cudaSuccess;
   return ok;
 }
 
@@ -1521,6 +1508,7 @@ static flow_ctx* create_impl(flow_arena* arena, const flow_grid_view* g, const f
   c->nnz = g->ia[nn + 1];
   if (cudaSetDevice(device) != cudaSuccess) return fail(c, FLOW_ERR_CUDA, "cudaSetDevice failed");
   cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device);
+  c->var[0] = default_node_variant(p->order, nn, c->nsm);
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess)
     return fail(c, FLOW_ERR_CUDA, "stream creation failed");
   cudaEventCreate(&c->ev0);
@@ -1641,10 +1629,17 @@ static flow_ctx* create_impl(flow_arena* arena, const flow_grid_view* g, const f
   }
   // k=2 stencils: node i uses gnsn[gnnsn[gnnsn1[i]+1] .. gnnsn[gnnsn1[i+1]])
   std::vector<int> st_ptr(nn + 2, 0), st_idx;
-  std::vector<double> st_w, U1, VT((size_t)(nn + 1) * 25, 0.), S((size_t)(nn + 1) * 5, 1.);
+  std::vector<double4> st_u;
+  std::vector<double2> st_uw;
+  std::vector<double> k2;
   int stencil_max = 0;
   c->has_stencils = p->order == 3 && all_st;
   if (c->has_stencils) {
+    k2.assign((size_t)(nn + 1) * kK2Words, 0.);
+    const size_t rows = (size_t)g->gnnsn[g->gnnsn1[nn + 1]];
+    st_idx.reserve(rows);
+    st_u.reserve(rows);
+    st_uw.reserve(rows);
     for (int i = 1; i <= nn; i++) {
       int a0 = g->gnnsn[g->gnnsn1[i] + 1], a1 = g->gnnsn[g->gnnsn1[i + 1]];
       int mrows = a1 - a0;
@@ -1658,14 +1653,25 @@ static flow_ctx* create_impl(flow_arena* arena, const flow_grid_view* g, const f
         double dx1 = g->x[2 * nb + 1] - g->x[2 * i + 1];
         double dist = sqrt(dx0 * dx0 + dx1 * dx1);
         st_idx.push_back(nb);
-        st_w.push_back(1.0 / pow(dist, 1.0));  // compute_derivatives.C:1470 (GEOM_WEIGHT 1)
+        // column 4 of U and the weight (compute_derivatives.C:1470, GEOM_WEIGHT 1)
+        st_uw.push_back(make_double2(0., 1.0 / pow(dist, 1.0)));
       }
+      // the first 5 columns of U row by row
       const double* Ui = g->svd_U + g->svd_off[i];
-      // the first 5 columns of U, re-laid row by row (U1[k][c] = U[c*m + k])
-      for (int k = 0; k < mrows; k++)
-        for (int q = 0; q < 5; q++) U1.push_back(Ui[q * mrows + k]);
-      for (int q = 0; q < 25; q++) VT[(size_t)i * 25 + q] = g->svd_VT[(size_t)i * 25 + q];
-      for (int q = 0; q < 5; q++) S[(size_t)i * 5 + q] = g->svd_S[(size_t)i * 5 + q];
+      for (int k = 0; k < mrows; k++) {
+        st_u.push_back(make_double4(Ui[k], Ui[mrows + k], Ui[2 * mrows + k], Ui[3 * mrows + k]));
+        st_uw[st_ptr[i] + k].x = Ui[4 * mrows + k];
+      }
+      double* rec = &k2[(size_t)i * kK2Words];
+      for (int q = 0; q < 5; q++) {
+        const double S = g->svd_S[(size_t)i * 5 + q];
+        rec[kK2S + q] = S;
+        // the reciprocal div_recip needs, NaN outside its range (pivot_recip)
+        const int ex = S == 0. || !std::isfinite(S) ? 9999 : std::ilogb(S);
+        rec[kK2R + q] = ex >= -400 && ex <= 400 ? 1.0 / S : std::nan("");
+        rec[kK2M + q] = g->moments[(size_t)i * 9 + q];
+      }
+      for (int q = 0; q < 25; q++) rec[kK2V + q] = g->svd_VT[(size_t)i * 25 + q];
     }
     st_ptr[nn + 1] = (int)st_idx.size();
   }
@@ -1713,13 +1719,10 @@ static flow_ctx* create_impl(flow_arena* arena, const flow_grid_view* g, const f
     if (g->xg_bedges) std::copy(g->xg_bedges, g->xg_bedges + xgb.size(), xgb.begin());
     if (g->xgn_bedges) std::copy(g->xgn_bedges, g->xgn_bedges + xgnb.size(), xgnb.begin());
     UP(xg_bedges, xgb); UP(xgn_bedges, xgnb);
-    std::vector<double> mo((size_t)(nn + 1) * 9, 0.);
-    if (g->moments) std::copy(g->moments, g->moments + mo.size(), mo.begin());
-    UP(moments, mo);
   }
   if (c->has_stencils) {
-    UP(st_ptr, st_ptr); UP(st_idx, st_idx); UP(st_w, st_w);
-    UP(svd_U1, U1); UP(svd_VT, VT); UP(svd_S, S);
+    UP(st_ptr, st_ptr); UP(st_idx, st_idx); UP(st_u, st_u); UP(st_uw, st_uw);
+    UP(k2, k2);
   }
 #undef UP
   if (!okk) return fail(c, carve_error(c), "device allocation or upload failed");

@@ -134,31 +134,122 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// A double4 of data the kernel does not write, in one 32-byte access (ALIGNED:
+// p on a 32-byte boundary) or as four values.
+template <bool ALIGNED>
+__device__ __forceinline__ double4 ldg_d4(const double* p) {
+  double4 v;
+  if (ALIGNED)
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+        : "l"(p));
+  else
+    v = make_double4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+  return v;
+}
+
+__device__ __forceinline__ double4 ldg_d4(const double4* p) {
+  return ldg_d4<true>(reinterpret_cast<const double*>(p));
+}
+
+// h of the k=2 derivatives (x = V S^-1 U^T b) of NV variables from the sums
+// acc over their node's stencil, and the point values; k2: the node's record.
+template <int NV>
+__device__ __forceinline__ void k2_solve(const double* k2, const double (*acc)[5],
+                                         const double* q0, double (*h)[5], double* pv) {
+  const double4 r0 = ldg_d4<true>(k2), r1 = ldg_d4<true>(k2 + 4), r2 = ldg_d4<true>(k2 + 8),
+                r3 = ldg_d4<true>(k2 + 12);
+  const double S[5] = {r0.x, r0.y, r0.z, r0.w, r1.x}, R[5] = {r1.y, r1.z, r1.w, r2.x, r2.y};
+  const double mo[5] = {r2.z, r2.w, r3.x, r3.y, r3.z};
+  double t[NV][5];
+  bool ok = true;
+#pragma unroll
+  for (int i = 0; i < NV; i++)
+#pragma unroll
+    for (int c = 0; c < 5; c++) {
+      t[i][c] = div_recip(acc[i][c], S[c], R[c]);
+      // a sum is never -0 (it starts at +0), and +0 / S is +0 either way
+      ok = ok && (div_range(acc[i][c]) || acc[i][c] == 0.) && R[c] == R[c];
+    }
+  if (!ok)
+#pragma unroll
+    for (int i = 0; i < NV; i++)
+#pragma unroll
+      for (int c = 0; c < 5; c++) t[i][c] = acc[i][c] / S[c];
+  double4 v = r3;
+#pragma unroll
+  for (int j = 0; j < 5; j++) {
+    double sum[NV];
+#pragma unroll
+    for (int c = 0; c < 5; c++) {
+      const int e = 5 * j + c;
+      if (e % 4 == 0) v = ldg_d4<true>(k2 + kK2V + e);
+      const double x = e % 4 == 0 ? v.x : e % 4 == 1 ? v.y : e % 4 == 2 ? v.z : v.w;
+#pragma unroll
+      for (int i = 0; i < NV; i++) sum[i] = (c == 0 ? 0. : sum[i]) + x * t[i][c];
+    }
+#pragma unroll
+    for (int i = 0; i < NV; i++) h[i][j] = sum[i];
+  }
+#pragma unroll
+  for (int i = 0; i < NV; i++)
+    pv[i] = q0[i] - mo[0] * h[i][0] - mo[1] * h[i][1] - mo[2] * h[i][2] * 0.5 -
+            mo[3] * h[i][3] * 0.5 - mo[4] * h[i][4];
+}
+
 // ---------------------------------------------------------------------------
 // Per node: cv_calc_eigenvalue_contribution (cv_calc.C:819-953) and the dt /
 // V/dt of build_matrix (init_memory.C:200-290); then the LSQ gradient
 // (gradient.C:382-403) or the k=2 derivatives (compute_derivatives.C:
 // 1438-1521); then the Venkatakrishnan limiter (limiter.C:594-906).
-// Four lanes per node, lane v owning conserved variable v: the gradient,
-// the k=2 derivatives and point value, and the limiter value of variable v
-// only involve variable v, and each lane accumulates its sums in the
-// reference's face / stencil order.  The wave-speed sum (all variables) is
-// formed by every lane of the quad from node constants computed once.
-// MINB: resident blocks per SM the compiler must allow (0: its own choice);
-// the autotuner picks the variant that runs fastest on a given mesh.
-// LIM: 0 venkat_fold; 1 venkat_fold_nz (no division of or by zero); 2 the
-// same, with the wave-speed face terms formed in the limiter's face loop (one
-// walk of the node's faces, more registers).  All give the same bits.
-template <int ORDER, int MINB, int LIM = 0>
+// 4 / NV lanes per node, a lane owning NV of the conserved variables: the
+// gradient, the k=2 derivatives and point value, and the limiter value of a
+// variable only involve that variable, and each lane accumulates its sums in
+// the reference's face / stencil order.  The wave-speed sum (all variables) is
+// formed by every lane of the node from node constants computed once.
+//
+// Latency-bound on chains of dependent loads (incidence list -> face record,
+// stencil -> neighbour state), with the FP64 pipe and the issue slots half
+// busy; so what helps is fewer instructions and more nodes in flight.  The
+// limiter finds each side's decisive face point by a scan and divides twice
+// for it (LimiterScan) instead of twice a point, records are read in 16 and
+// 32-byte accesses (a stencil row in two, a node's V^T, S and moments in 11),
+// the five divisions by the singular values use their reciprocals, and with
+// NV = 2 the geometry is loaded and its products formed for two variables at
+// once.  MINB: resident blocks per SM the compiler must allow (how many
+// registers a lane may hold); MERGED: the wave-speed face terms formed in the
+// limiter's face loop (one walk of the node's faces, more registers).  Which
+// combination is fastest depends on the mesh (node_kernel lists them, the
+// autotuner picks); all give the same bits.  Best of them against the best
+// before (division a point, 8-byte loads), us: k=2 11k nodes 58 -> 26, 65k
+// 109 -> 77, 181k 248 -> 170 (2.3 TB/s of compulsory bytes), 496k 617 -> 418;
+// k=1 26k 22.5 -> 21.3, 496k 209 -> 179.
+template <int ORDER, int MINB, bool MERGED, int NV>
 __global__ void __launch_bounds__(128, MINB) k_node_prepare4(DevMesh m, DevState s, StepArgs a) {
   if (*s.stop) return;  // the run has converged
+  constexpr int LANES = 4 / NV;  // of a node
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = (tid >> 2) + 1, v = tid & 3;
-  const int qbase = threadIdx.x & ~3 & 31;
-  const unsigned qmask = 0xFu << qbase;
-  if (n > m.nn) return;  // whole quads leave together
-  const double4 q4 = reinterpret_cast<const double4*>(s.nQ)[n];
-  const double q0v = v == 0 ? q4.x : v == 1 ? q4.y : v == 2 ? q4.z : q4.w;
+  const int n = tid / LANES + 1, l = tid % LANES, v0 = NV * l;
+  const int base = threadIdx.x & 31 & ~(LANES - 1);
+  const unsigned mask = ((1u << LANES) - 1u) << base;
+  if (n > m.nn) return;  // a node's lanes leave together
+  const double4 q4 = ldg_d4<true>(s.nQ + 4 * (long)n);
+  double q0[NV];
+#pragma unroll
+  for (int i = 0; i < NV; i++) {
+    const int v = v0 + i;
+    q0[i] = v == 0 ? q4.x : v == 1 ? q4.y : v == 2 ? q4.z : q4.w;
+  }
+  // variables v0 .. v0+NV-1 of node j
+  auto load_q = [&](int j, double* q) {
+    if (NV == 1) {
+      q[0] = __ldg(s.nQ + 4 * (long)j + v0);
+    } else {
+      const double2 x = __ldg(reinterpret_cast<const double2*>(s.nQ + 4 * (long)j) + l);
+      q[0] = x.x;
+      q[NV - 1] = x.y;
+    }
+  };
 
   // ---- wave-speed sum (cv_calc.C:819-953): node constants first ----
   double uu, vv, cs;
@@ -190,128 +281,172 @@ __global__ void __launch_bounds__(128, MINB) k_node_prepare4(DevMesh m, DevState
       if (!isfinite(w)) bad = 1;
       ev += (w * xn[2]);
     }
-    if (v == 0) {
+    if (l == 0) {
       const double dt = s.scalars[3] * (m.cv_area[n] / ev);  // cfl of the step (step_args_body)
       s.dt[n] = dt;
       if (bad) atomicOr(s.status, ERR_EIGEN);
       if (dt <= 0. || !isfinite(dt)) atomicOr(s.status, ERR_DT);
     }
   };
-  // LIM 2 with the limiter on: the face terms are summed inside the
+  // MERGED with the limiter on: the face terms are summed inside the
   // limiter's pass over the same faces (the same order), one walk of the
   // node's incidence list instead of two
-  const bool merged = LIM == 2 && a.do_lim;
+  const bool merged = MERGED && a.do_lim;
   if (!merged) {
     node_consts(q4);
     #pragma unroll 4
-    for (int k = s0; k < s1; k++) wave_term(m.sub_geo[m.nsub[k] >> 1]);
+    for (int k = s0; k < s1; k++) wave_term(ldg_d4(m.sub_geo + (m.nsub[k] >> 1)));
     finish_wave();
   }
   if (!a.do_grad && !a.do_derivs && !a.do_lim) return;
 
-  // ---- 1-ring min/max and the k=1 LSQ gradient of variable v ----
-  double qmin = q0v, qmax = q0v, g0 = 0., g1 = 0.;
+  // ---- 1-ring min/max and the k=1 LSQ gradient of the lane's variables ----
+  double qmin[NV], qmax[NV], g0[NV], g1[NV];
+#pragma unroll
+  for (int i = 0; i < NV; i++) {
+    qmin[i] = qmax[i] = q0[i];
+    g0[i] = g1[i] = 0.;
+  }
   const int e0 = m.nedg_ptr[n], e1 = m.nedg_ptr[n + 1];
   #pragma unroll 4
   for (int k = e0; k < e1; k++) {
     // the neighbour straight from the node's incidence list (nedg_nbr), so
     // its state is one dependent load away, not two
-    const double qo = s.nQ[4 * (long)m.nedg_nbr[k] + v];
-    qmin = qmin <= qo ? qmin : qo;
-    qmax = qmax >= qo ? qmax : qo;
+    double qo[NV];
+    load_q(m.nedg_nbr[k], qo);
+    double4 w;
+    int side = 0;
     if (ORDER == 1 && a.do_grad) {
       const int ed = m.nedg[k];
-      const int e = ed >> 1, side = ed & 1;
-      const double4 w = m.edge_w[e];
-      const double dq = side ? (q0v - qo) : (qo - q0v);  // nQ[R] - nQ[L]
-      if (side == 0) {
-        g0 += w.x * dq;
-        g1 += w.y * dq;
-      } else {
-        g0 -= w.z * dq;
-        g1 -= w.w * dq;
+      side = ed & 1;
+      w = ldg_d4(m.edge_w + (ed >> 1));
+    }
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+      qmin[i] = qmin[i] <= qo[i] ? qmin[i] : qo[i];
+      qmax[i] = qmax[i] >= qo[i] ? qmax[i] : qo[i];
+      if (ORDER == 1 && a.do_grad) {
+        const double dq = side ? (q0[i] - qo[i]) : (qo[i] - q0[i]);  // nQ[R] - nQ[L]
+        if (side == 0) {
+          g0[i] += w.x * dq;
+          g1[i] += w.y * dq;
+        } else {
+          g0[i] -= w.z * dq;
+          g1[i] -= w.w * dq;
+        }
       }
     }
   }
   if (ORDER == 1 && a.do_grad)
-    reinterpret_cast<double2*>(s.grad + 8 * (long)n)[v] = make_double2(g0, g1);
+#pragma unroll
+    for (int i = 0; i < NV; i++)
+      reinterpret_cast<double2*>(s.grad + 8 * (long)n)[v0 + i] = make_double2(g0[i], g1[i]);
 
-  // ---- k=2: x = V S^-1 U^T b of variable v ----
-  double h[5], pv = 0.;
+  // ---- k=2: x = V S^-1 U^T b of the lane's variables ----
+  double h[NV][5], pv[NV];
   if (ORDER == 3 && a.do_derivs) {
     const int t0 = m.st_ptr[n], t1 = m.st_ptr[n + 1];
-    const int mrows = t1 - t0;
-    const double* U = m.svd_U1 + 5 * (long)t0;  // row k: U[k][0..4], contiguous
-    double acc[5] = {0., 0., 0., 0., 0.};
+    double acc[NV][5];
+#pragma unroll
+    for (int i = 0; i < NV; i++)
+#pragma unroll
+      for (int c = 0; c < 5; c++) acc[i][c] = 0.;
 #pragma unroll 4
-    for (int k = 0; k < mrows; k++) {
-      const int nb = m.st_idx[t0 + k];
-      const double bv = m.st_w[t0 + k] * (s.nQ[4 * (long)nb + v] - q0v);
+    for (int k = t0; k < t1; k++) {
+      double qo[NV];
+      load_q(m.st_idx[k], qo);
+      const double4 u = ldg_d4(m.st_u + k);
+      const double2 uw = __ldg(m.st_uw + k);
 #pragma unroll
-      for (int c = 0; c < 5; c++) acc[c] += bv * U[5 * k + c];
+      for (int i = 0; i < NV; i++) {
+        const double bv = uw.y * (qo[i] - q0[i]);
+        acc[i][0] += bv * u.x;
+        acc[i][1] += bv * u.y;
+        acc[i][2] += bv * u.z;
+        acc[i][3] += bv * u.w;
+        acc[i][4] += bv * uw.x;
+      }
     }
-      const double* VT = m.svd_VT + 25 * (long)n;
-    const double* S = m.svd_S + 5 * (long)n;
-    double t1v[5];
+    k2_solve<NV>(m.k2 + kK2Words * (long)n, acc, q0, h, pv);
+    double* hd = s.hess5 + 20 * (long)n + 5 * v0;
 #pragma unroll
-    for (int c = 0; c < 5; c++) t1v[c] = acc[c] / S[c];
+    for (int i = 0; i < NV; i++) {
 #pragma unroll
-    for (int j = 0; j < 5; j++) {
-      double sum = 0.;
-#pragma unroll
-      for (int c = 0; c < 5; c++) sum += VT[j * 5 + c] * t1v[c];
-      h[j] = sum;
+      for (int c = 0; c < 5; c++) hd[5 * i + c] = h[i][c];
+      s.pv[4 * (long)n + v0 + i] = pv[i];
     }
-    const double* mo = m.moments + 9 * (long)n;
-    pv = q0v - mo[0] * h[0] - mo[1] * h[1] - mo[2] * h[2] * 0.5 - mo[3] * h[3] * 0.5 -
-         mo[4] * h[4];
-    double* hd = s.hess5 + 20 * (long)n + 5 * v;
-#pragma unroll
-    for (int c = 0; c < 5; c++) hd[c] = h[c];
-    s.pv[4 * (long)n + v] = pv;
   }
 
   if (!a.do_lim) return;
-  // ---- Venkatakrishnan bound of variable v over every face point ----
-  double ph = 1.0;
+  // ---- Venkatakrishnan bound of the lane's variables over every face point ----
+  double ph[NV];
+#pragma unroll
+  for (int i = 0; i < NV; i++) ph[i] = 1.0;
   const double xn0 = m.x[2 * n], xn1 = m.x[2 * n + 1];
   // the node constants formed again here rather than held through the
   // gradient and stencil loops (the same expressions: the same bits)
-  if (merged) node_consts(reinterpret_cast<const double4*>(s.nQ)[n]);
-  #pragma unroll 4
-  for (int k = s0; k < s1; k++) {
-    const int sd = m.nsub[k];
-    const int sub = sd >> 1, side = sd & 1;
-    if (merged) wave_term(m.sub_geo[sub]);
-    if (ORDER == 1) {
-      const double4 d = m.sub_dx[sub];
-      const double dx0 = side ? d.z : d.x, dx1 = side ? d.w : d.y;
-      const double qr = q0v + (g0 * dx0 + g1 * dx1);
-      ph = venkat_fold_lim<LIM>(ph, qr, q0v, qmin, qmax);
-    } else {
-      const double* xg = m.sub_xg + 6 * (long)sub;
+  if (merged) node_consts(ldg_d4<true>(s.nQ + 4 * (long)n));
+  // every face point's reconstructed values, in face order
+  auto face_points = [&](bool wave, auto&& point) {
+#pragma unroll 2
+    for (int k = s0; k < s1; k++) {
+      const int sd = m.nsub[k];
+      const int sub = sd >> 1, side = sd & 1;
+      if (wave) wave_term(ldg_d4(m.sub_geo + sub));
+      if (ORDER == 1) {
+        const double4 d = ldg_d4(m.sub_dx + sub);
+        const double dx0 = side ? d.z : d.x, dx1 = side ? d.w : d.y;
 #pragma unroll
-      for (int gpt = 0; gpt < 3; gpt++) {
-        const double dx0 = xg[2 * gpt] - xn0, dx1 = xg[2 * gpt + 1] - xn1;
-        double qr = pv;
-        qr += (h[0] * dx0 + h[1] * dx1 + h[2] * dx0 * dx0 * 0.5 + h[3] * dx1 * dx1 * 0.5 +
-               h[4] * dx0 * dx1);
-        ph = venkat_fold_lim<LIM>(ph, qr, q0v, qmin, qmax);
+        for (int i = 0; i < NV; i++) point(i, q0[i] + (g0[i] * dx0 + g1[i] * dx1));
+      } else {
+        const double2* xg = reinterpret_cast<const double2*>(m.sub_xg + 6 * (long)sub);
+#pragma unroll
+        for (int gpt = 0; gpt < 3; gpt++) {
+          const double2 x = __ldg(xg + gpt);
+          const double dx0 = x.x - xn0, dx1 = x.y - xn1;
+#pragma unroll
+          for (int i = 0; i < NV; i++) {
+            double qr = pv[i];
+            qr += (h[i][0] * dx0 + h[i][1] * dx1 + h[i][2] * dx0 * dx0 * 0.5 +
+                   h[i][3] * dx1 * dx1 * 0.5 + h[i][4] * dx0 * dx1);
+            point(i, qr);
+          }
+        }
       }
+    }
+  };
+  {
+    LimiterScan scan[NV];
+    face_points(merged, [&](int i, double qr) { scan[i].add(qr - q0[i]); });
+    bool settled = true;
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+      const double a_up = qmax[i] - q0[i], a_down = qmin[i] - q0[i];
+      settled = settled && scan[i].settled(a_up, a_down);
+      ph[i] = scan[i].phi(a_up, a_down);
+    }
+    if (!settled) {
+#pragma unroll
+      for (int i = 0; i < NV; i++) ph[i] = 1.0;
+      face_points(false, [&](int i, double qr) {
+        ph[i] = venkat_fold(ph[i], qr, q0[i], qmin[i], qmax[i]);
+      });
     }
   }
   if (merged) finish_wave();
   // min over the variables in order 0..3 (limiter.C:895-906)
-  const double p1 = __shfl_sync(qmask, ph, qbase + 1);
-  const double p2 = __shfl_sync(qmask, ph, qbase + 2);
-  const double p3 = __shfl_sync(qmask, ph, qbase + 3);
-  double pmin = ph;
-  pmin = pmin <= p1 ? pmin : p1;
-  pmin = pmin <= p2 ? pmin : p2;
-  pmin = pmin <= p3 ? pmin : p3;
-  const double out = v == 0 ? pmin : ph;
-  reinterpret_cast<double2*>(s.phi + 8 * (long)n)[v] = make_double2(out, out);
-  if (out < 0.0 || out > 1.0) atomicOr(s.status, ERR_LIMITER);
+  double pmin = ph[0];
+#pragma unroll
+  for (int v = 1; v < 4; v++) {
+    const double p = v < NV ? ph[v % NV] : __shfl_sync(mask, ph[v % NV], base + v / NV);
+    pmin = pmin <= p ? pmin : p;
+  }
+#pragma unroll
+  for (int i = 0; i < NV; i++) {
+    const double out = v0 + i == 0 ? pmin : ph[i];
+    reinterpret_cast<double2*>(s.phi + 8 * (long)n)[v0 + i] = make_double2(out, out);
+    if (out < 0.0 || out > 1.0) atomicOr(s.status, ERR_LIMITER);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -335,8 +470,7 @@ __device__ __forceinline__ double hshfl(double x, unsigned mask, int lane) {
   return __shfl_sync(mask, x, lane);
 }
 
-// LIM: the limiter's fold, as in k_node_prepare4.
-template <int ORDER, int LIM = 0>
+template <int ORDER>
 __global__ void __launch_bounds__(128) k_node_prepare16(DevMesh m, DevState s, StepArgs a) {
   if (*s.stop) return;  // the run has converged
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -357,7 +491,7 @@ __global__ void __launch_bounds__(128) k_node_prepare16(DevMesh m, DevState s, S
   for (int base = s0; base < s1; base += 16) {
     double term = 0.;
     if (base + l < s1) {
-      const double4 gg = m.sub_geo[m.nsub[base + l] >> 1];
+      const double4 gg = ldg_d4(m.sub_geo + (m.nsub[base + l] >> 1));
       const double theta = uu * gg.x + vv * gg.y;
       const double tpc = fabs(theta + cs), tmc = fabs(theta - cs);
       const double w = tpc >= tmc ? tpc : tmc;
@@ -403,7 +537,7 @@ __global__ void __launch_bounds__(128) k_node_prepare16(DevMesh m, DevState s, S
       qmax = qmax >= qo ? qmax : qo;
     }
     if (grad) {
-      const double4 w = m.edge_w[ed >> 1];
+      const double4 w = ldg_d4(m.edge_w + (ed >> 1));
       const double dq = side ? (q0v - qo) : (qo - q0v);  // nQ[R] - nQ[L]
       if (side == 0) gsum += (g == 0 ? w.x : w.y) * dq;
       else gsum -= (g == 0 ? w.z : w.w) * dq;
@@ -420,36 +554,24 @@ __global__ void __launch_bounds__(128) k_node_prepare16(DevMesh m, DevState s, S
   double h[5] = {0., 0., 0., 0., 0.}, pv = 0.;
   if (ORDER == 3 && a.do_derivs) {
     const int t0 = m.st_ptr[n], t1 = m.st_ptr[n + 1];
-    const int mrows = t1 - t0;
-    const double* U = m.svd_U1 + 5 * (long)t0;
     double accA = 0., accB = 0.;
 #pragma unroll 4
-    for (int k = 0; k < mrows; k++) {
-      const int nb = m.st_idx[t0 + k];
-      const double bv = m.st_w[t0 + k] * (s.nQ[4 * (long)nb + v] - q0v);
-      accA += bv * U[5 * k + g];
-      if (g == 0) accB += bv * U[5 * k + 4];
+    for (int k = t0; k < t1; k++) {
+      const int nb = m.st_idx[k];
+      const double2 uw = m.st_uw[k];
+      const double bv = uw.y * (s.nQ[4 * (long)nb + v] - q0v);
+      accA += bv * reinterpret_cast<const double*>(m.st_u + k)[g];
+      if (g == 0) accB += bv * uw.x;
     }
-    const double* S = m.svd_S + 5 * (long)n;
-    const double tA = accA / S[g];
-    const double tB = g == 0 ? accB / S[4] : 0.;
-    double t1v[5];
-    t1v[0] = hshfl(tA, hmask, hbase + v);
-    t1v[1] = hshfl(tA, hmask, hbase + 4 + v);
-    t1v[2] = hshfl(tA, hmask, hbase + 8 + v);
-    t1v[3] = hshfl(tA, hmask, hbase + 12 + v);
-    t1v[4] = hshfl(tB, hmask, hbase + v);
-    const double* VT = m.svd_VT + 25 * (long)n;
+    double acc[1][5], hh[1][5];
+    acc[0][0] = hshfl(accA, hmask, hbase + v);
+    acc[0][1] = hshfl(accA, hmask, hbase + 4 + v);
+    acc[0][2] = hshfl(accA, hmask, hbase + 8 + v);
+    acc[0][3] = hshfl(accA, hmask, hbase + 12 + v);
+    acc[0][4] = hshfl(accB, hmask, hbase + v);
+    k2_solve<1>(m.k2 + kK2Words * (long)n, acc, &q0v, hh, &pv);
 #pragma unroll
-    for (int j = 0; j < 5; j++) {
-      double sum = 0.;
-#pragma unroll
-      for (int c = 0; c < 5; c++) sum += VT[j * 5 + c] * t1v[c];
-      h[j] = sum;
-    }
-    const double* mo = m.moments + 9 * (long)n;
-    pv = q0v - mo[0] * h[0] - mo[1] * h[1] - mo[2] * h[2] * 0.5 - mo[3] * h[3] * 0.5 -
-         mo[4] * h[4];
+    for (int c = 0; c < 5; c++) h[c] = hh[0][c];
     if (g == 0) {
       double* hd = s.hess5 + 20 * (long)n + 5 * v;
 #pragma unroll
@@ -461,31 +583,27 @@ __global__ void __launch_bounds__(128) k_node_prepare16(DevMesh m, DevState s, S
   if (!a.do_lim) return;
   // ---- Venkatakrishnan bound of variable v over every face point ----
   const double xn0 = m.x[2 * n], xn1 = m.x[2 * n + 1];
-  auto fold_faces = [&](double mn, double mx, int first, int stride, int& sawnan) {
-    double ph = 1.0;
+  auto face_points = [&](int first, int stride, auto&& point) {
     for (int k = s0 + first; k < s1; k += stride) {
       const int sd = m.nsub[k];
       const int sub = sd >> 1, side = sd & 1;
       if (ORDER == 1) {
-        const double4 d = m.sub_dx[sub];
+        const double4 d = ldg_d4(m.sub_dx + sub);
         const double dx0 = side ? d.z : d.x, dx1 = side ? d.w : d.y;
-        const double qr = q0v + (g0 * dx0 + g1 * dx1);
-        ph = venkat_fold_lim<LIM>(ph, qr, q0v, mn, mx);
-        if (ph != ph) sawnan = 1;
+        point(q0v + (g0 * dx0 + g1 * dx1));
       } else {
-        const double* xg = m.sub_xg + 6 * (long)sub;
+        const double2* xg = reinterpret_cast<const double2*>(m.sub_xg + 6 * (long)sub);
 #pragma unroll
         for (int gpt = 0; gpt < 3; gpt++) {
-          const double dx0 = xg[2 * gpt] - xn0, dx1 = xg[2 * gpt + 1] - xn1;
+          const double2 x = xg[gpt];
+          const double dx0 = x.x - xn0, dx1 = x.y - xn1;
           double qr = pv;
           qr += (h[0] * dx0 + h[1] * dx1 + h[2] * dx0 * dx0 * 0.5 + h[3] * dx1 * dx1 * 0.5 +
                  h[4] * dx0 * dx1);
-          ph = venkat_fold_lim<LIM>(ph, qr, q0v, mn, mx);
-          if (ph != ph) sawnan = 1;
+          point(qr);
         }
       }
     }
-    return ph;
   };
   // this variable's 1-ring min/max from the four groups
   double mn = qmin, mx = qmax;
@@ -496,16 +614,25 @@ __global__ void __launch_bounds__(128) k_node_prepare16(DevMesh m, DevState s, S
     mn = mn <= omn ? mn : omn;
     mx = mx >= omx ? mx : omx;
   }
-  int sawnan = 0;
-  double ph = fold_faces(mn, mx, g, 4, sawnan);
-  double pg = ph;
+  double pg = 1.0;
+  bool in_order = nan;  // this lane's fold depends on the order of the points
+  {
+    const double a_up = mx - q0v, a_down = mn - q0v;
+    LimiterScan own;
+    face_points(g, 4, [&](double qr) { own.add(qr - q0v); });
+    LimiterScan scan = own;
 #pragma unroll
-  for (int gg = 1; gg < 4; gg++) {
-    const double o = hshfl(ph, hmask, hbase + ((g + gg) & 3) * 4 + v);
-    pg = pg <= o ? pg : o;
+    for (int gg = 1; gg < 4; gg++) {
+      const int from = hbase + ((g + gg) & 3) * 4 + v;
+      auto f = [&](float x) { return __shfl_sync(hmask, x, from); };
+      scan.merge(hshfl(own.up, hmask, from), f(own.up1), f(own.up2), hshfl(own.down, hmask, from),
+                 f(own.down1), f(own.down2), __shfl_sync(hmask, (int)own.tiny, from));
+    }
+    in_order = in_order || !scan.settled(a_up, a_down);
+    if (!in_order) pg = scan.phi(a_up, a_down);
   }
-  if (__any_sync(hmask, nan | sawnan)) {
-    // a NaN makes the folds order-dependent: the reference's order throughout
+  if (__any_sync(hmask, in_order)) {
+    // the points in the reference's order throughout
     mn = q0v;
     mx = q0v;
     for (int k = e0; k < e1; k++) {
@@ -513,8 +640,8 @@ __global__ void __launch_bounds__(128) k_node_prepare16(DevMesh m, DevState s, S
       mn = mn <= qo ? mn : qo;
       mx = mx >= qo ? mx : qo;
     }
-    int unused = 0;
-    pg = fold_faces(mn, mx, 0, 1, unused);
+    pg = 1.0;
+    face_points(0, 1, [&](double qr) { pg = venkat_fold(pg, qr, q0v, mn, mx); });
   }
   // min over the variables in order 0..3 (limiter.C:895-906)
   const double p1 = hshfl(pg, hmask, hbase + 1);
@@ -694,31 +821,22 @@ __global__ void __launch_bounds__(128) k_node_stage(DevMesh m, DevState s, StepA
   double h[5], pv = 0.;
   if (derivs) {
     const int t0 = m.st_ptr[n], t1 = m.st_ptr[n + 1];
-    const int mrows = t1 - t0;
-    const double* U = m.svd_U1 + 5 * (long)t0;
-    double acc[5] = {0., 0., 0., 0., 0.};
+    double acc[1][5] = {{0., 0., 0., 0., 0.}}, hh[1][5];
 #pragma unroll 4
-    for (int k = 0; k < mrows; k++) {
-      const double qn = reinterpret_cast<const double*>(&s_nqs[t0 - R0 + k])[v];
-      const double bv = m.st_w[t0 + k] * (qn - q0v);
-#pragma unroll
-      for (int c = 0; c < 5; c++) acc[c] += bv * U[5 * k + c];
+    for (int k = t0; k < t1; k++) {
+      const double qn = reinterpret_cast<const double*>(&s_nqs[k - R0])[v];
+      const double4 u = ldg_d4(m.st_u + k);
+      const double2 uw = m.st_uw[k];
+      const double bv = uw.y * (qn - q0v);
+      acc[0][0] += bv * u.x;
+      acc[0][1] += bv * u.y;
+      acc[0][2] += bv * u.z;
+      acc[0][3] += bv * u.w;
+      acc[0][4] += bv * uw.x;
     }
-    const double* VT = m.svd_VT + 25 * (long)n;
-    const double* S = m.svd_S + 5 * (long)n;
-    double t1v[5];
+    k2_solve<1>(m.k2 + kK2Words * (long)n, acc, &q0v, hh, &pv);
 #pragma unroll
-    for (int c = 0; c < 5; c++) t1v[c] = acc[c] / S[c];
-#pragma unroll
-    for (int j = 0; j < 5; j++) {
-      double sum = 0.;
-#pragma unroll
-      for (int c = 0; c < 5; c++) sum += VT[j * 5 + c] * t1v[c];
-      h[j] = sum;
-    }
-    const double* mo = m.moments + 9 * (long)n;
-    pv = q0v - mo[0] * h[0] - mo[1] * h[1] - mo[2] * h[2] * 0.5 - mo[3] * h[3] * 0.5 -
-         mo[4] * h[4];
+    for (int c = 0; c < 5; c++) h[c] = hh[0][c];
     double* hd = s.hess5 + 20 * (long)n + 5 * v;
 #pragma unroll
     for (int c = 0; c < 5; c++) hd[c] = h[c];
@@ -2309,20 +2427,6 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
   double out = sh[0];
   __syncthreads();
   return out;
-}
-
-// A double4 of data the kernel does not write, in one 32-byte access (ALIGNED:
-// p on a 32-byte boundary) or as four values.
-template <bool ALIGNED>
-__device__ __forceinline__ double4 ldg_d4(const double* p) {
-  double4 v;
-  if (ALIGNED)
-    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-        : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
-        : "l"(p));
-  else
-    v = make_double4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
-  return v;
 }
 
 // |b - Ax|^2 of the rows by quads of lanes, lane q owning component q: row j's

@@ -13,6 +13,10 @@
 
 namespace flow {
 
+// A node's record of the k=2 derivatives: the singular values, their
+// reciprocals (pivot_recip), the first five moments, V^T row by row.
+constexpr int kK2Words = 44, kK2S = 0, kK2R = 5, kK2M = 10, kK2V = 16;
+
 struct DevMesh {
   int nn;        // real nodes (1..nn)
   int ng;        // ghost nodes (nn+1..nn+ng)
@@ -54,14 +58,12 @@ struct DevMesh {
   const double* x;
   const double* cv_area;
   const int* node_order;
-  const double* moments;   // 9 per node
   // k=2 stencil and factors
   const int* st_ptr;
   const int* st_idx;
-  const double* st_w;
-  const double* svd_U1;    // per node: first 5 columns of U, row by row, offset 5*st_ptr[i]
-  const double* svd_VT;    // 25 per node
-  const double* svd_S;     // 5 per node
+  const double4* st_u;     // per stencil row: columns 0..3 of U
+  const double2* st_uw;    // per stencil row: column 4 of U, the row's weight
+  const double* k2;        // kK2Words per node (kK2S ..): S, 1/S, moments, V^T
 };
 
 // Precision form: FP32 off-diagonal blocks and LU factors laid out in

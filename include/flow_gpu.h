@@ -420,22 +420,18 @@ long flow_launch_count(flow_ctx *ctx);
 double flow_last_device_ms(flow_ctx *ctx);
 
 /* ---- Autotuner (no counterpart in the reference) -------------------------
- * k_node_prepare4 comes in five variants, k_subedge_flux in three; the
- * results are bit-identical, the speed depends on the mesh.  Variants 0..2
- * of both set the minimum resident blocks per SM the compiler must allow
- * (how many registers a thread may hold); node variant 3 is the staged
- * kernel (a CTA of 32 nodes copies its incidence and stencil slices, then
- * gathers every face record and neighbour state into shared memory with
- * asynchronous copies before the arithmetic), offered where its shared
- * memory fits the mesh; node variant 4 gives each node 16 lanes instead of
- * 4 (its stencil columns, gradient components and face points spread over
- * them, every sum still in the reference's order); node variants 5, 6 and
- * 7 are variants 0, 1 and 4 with a limiter that divides no zero and by no
- * zero (a face point whose reconstruction equals the node's value, or whose
- * bound is the node's own value, folds in the value the reference's
- * quotients give there without dividing), variant 5 also forming the
- * wave-speed face terms in the limiter's walk over the faces; every variant
- * gives the same bits.
+ * The node kernel comes in eight variants, k_subedge_flux in three; the
+ * results are bit-identical, the speed depends on the mesh.  Node variants 0,
+ * 1, 2, 4, 5 and 6 differ in the registers a thread may hold, in how many of
+ * the conserved variables a lane owns and in whether the wave-speed sum walks
+ * the faces with the limiter; 3 is the staged kernel (a CTA of 32 nodes copies
+ * its incidence and stencil slices, then gathers every face record and
+ * neighbour state into shared memory with asynchronous copies before the
+ * arithmetic), offered where its shared memory fits the mesh; 7 gives each
+ * node 16 lanes (its stencil columns, gradient components and face points
+ * spread over them, every sum still in the reference's order).  Flux variants
+ * 0..2 differ in the registers a thread may hold.  A new context starts with
+ * a node variant chosen by its order and size, and flux variant 0.
  * flow_autotune times each variant over `steps`
  * pseudo-time steps from step index `ts` (CUDA events, after one warm-up
  * step), keeps the fastest, and puts the solution state back as it was
