@@ -480,27 +480,18 @@ int launch_residuals(flow_ctx* c, const StepArgs& a, int jac) {
   const bool approx = jac && c->jac_mode != 0 && c->precision != 0;
   {
     Timed t(c, 1);
-    int nbs = grid_blocks(c->ns, 128);
-    if (a.recon == 1) {
-      launch_flux_variant(c->var[1], [&](auto V) {
-        if (approx) k_subedge_flux<1, true, V.value, 1><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a);
-        else if (jac) k_subedge_flux<1, true, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a);
-        else k_subedge_flux<1, false, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a);
-      });
-    } else {
-      launch_flux_variant(c->var[1], [&](auto V) {
-        if (approx) k_subedge_flux<0, true, V.value, 1><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a);
-        else if (jac) k_subedge_flux<0, true, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a);
-        else k_subedge_flux<0, false, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a);
-      });
-    }
-    rc |= launch_check(c);
-  }
-  int nbb = grid_blocks(c->nbe, 128);
-  if (nbb > 0) {
-    Timed t(c, 2);
-    if (jac) k_boundary<true><<<nbb, 128, 0, c->stream>>>(c->m, c->s, a);
-    else k_boundary<false><<<nbb, 128, 0, c->stream>>>(c->m, c->s, a);
+    const int nbs = grid_blocks(c->ns, 128) + grid_blocks(c->nbe, 128);
+    launch_flux_variant(c->var[1], [&](auto V) {
+      if (a.recon == 1) {
+        if (approx) k_subedge_flux<1, true, V.value, 1><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, 1);
+        else if (jac) k_subedge_flux<1, true, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, 1);
+        else k_subedge_flux<1, false, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, 1);
+      } else {
+        if (approx) k_subedge_flux<0, true, V.value, 1><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, 1);
+        else if (jac) k_subedge_flux<0, true, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, 1);
+        else k_subedge_flux<0, false, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, 1);
+      }
+    });
     rc |= launch_check(c);
   }
   {
@@ -554,10 +545,13 @@ ChunkDfKernel chunk_df_kernel(const ChunkTables& ct, int dir) {
 // forward/backward, each followed by the b-Ax RMS that may stop the loop.
 // Precision form: p->subits multicolour FP32 sweeps from dQ = 0, colours
 // ascending on forward sweeps and descending on backward ones; no b-Ax RMS.
-int launch_linear_solve_mixed(flow_ctx* c, const flow_params* p) {
+// cleared: the assembly before this left the iterate zero (StepArgs::zero_iterate).
+int launch_linear_solve_mixed(flow_ctx* c, const flow_params* p, bool cleared) {
   int rc = 0;
-  cudaMemsetAsync(c->s.dQ, 0, sizeof(double) * 4 * (c->nn + 1), c->stream);
-  cudaMemsetAsync(c->mt.dq32, 0, sizeof(float) * 4 * (c->nn + 1), c->stream);
+  // the last sweep writes every row of the FP64 dQ
+  if (!cleared || p->subits < 1)
+    cudaMemsetAsync(c->s.dQ, 0, sizeof(double) * 4 * (c->nn + 1), c->stream);
+  if (!cleared) cudaMemsetAsync(c->mt.dq32, 0, sizeof(float) * 4 * (c->nn + 1), c->stream);
   if (c->precision == 3) {
     // coloured chunks of the reference order, in-place FP32 iterate
     const ChunkTables& ct = c->ct;
@@ -608,12 +602,11 @@ int launch_linear_solve_mixed(flow_ctx* c, const flow_params* p) {
   }
   if (c->precision == 2) {
     // reference row order: dispenser sweeps on ping-pong FP32 iterates
-    cudaMemsetAsync(c->s.skip, 0, sizeof(int), c->stream);
+    if (!cleared) cudaMemsetAsync(c->s.skip, 0, sizeof(int), c->stream);
     const long max_spin = 1L << 21;
     for (int it = 0; it < p->subits; it++) {
       Timed t(c, 4);
       const int last = it == p->subits - 1;
-      cudaMemsetAsync(c->s.counter, 0, sizeof(unsigned), c->stream);
       k_prepare_sweep32<<<grid_blocks(4 * (c->nn + 1), 256), 256, 0, c->stream>>>(
           c->s, c->mt.dq32, c->mt.dq32b, 4 * (c->nn + 1));
       rc |= launch_check(c);
@@ -646,11 +639,13 @@ int launch_linear_solve_mixed(flow_ctx* c, const flow_params* p) {
   return rc;
 }
 
-int launch_linear_solve(flow_ctx* c, const flow_params* p, bool final_rms) {
-  if (c->precision != 0) return launch_linear_solve_mixed(c, p);
+int launch_linear_solve(flow_ctx* c, const flow_params* p, bool final_rms, bool cleared) {
+  if (c->precision != 0) return launch_linear_solve_mixed(c, p, cleared);
   int rc = 0;
-  cudaMemsetAsync(c->s.dQ, 0, sizeof(double) * 4 * (c->nn + 1), c->stream);
-  cudaMemsetAsync(c->s.skip, 0, sizeof(int), c->stream);
+  if (!cleared) {
+    cudaMemsetAsync(c->s.dQ, 0, sizeof(double) * 4 * (c->nn + 1), c->stream);
+    cudaMemsetAsync(c->s.skip, 0, sizeof(int), c->stream);
+  }
   const long max_spin = 1L << 21;  // ~0.1-0.2 s per wait at most
   for (int it = 0; it < p->subits; it++) {
     {
@@ -672,7 +667,6 @@ int launch_linear_solve(flow_ctx* c, const flow_params* p, bool final_rms) {
       } else {
         // results go to the other dQ buffer, pre-filled with the not-ready
         // pattern; the buffers swap roles afterwards
-        cudaMemsetAsync(c->s.counter, 0, sizeof(unsigned), c->stream);
         double* dq_new = c->s.dQ2;
         k_prepare_sweep<<<grid_blocks(4 * (c->nn + 1), 256), 256, 0, c->stream>>>(
             c->s, c->s.dQ, dq_new, 4 * (c->nn + 1));
@@ -731,24 +725,29 @@ int begin_flags(const flow_ctx* c, const flow_params* p, const StepArgs& a) {
 // One solve() call (solve.C:44-933), device-only.  device_ts: the step index
 // advances on the device (for captured chunks of steps; ts then only selects
 // the order phase, which must be the same for every step of the chunk) and
-// the run's first step is recognised on the device.
+// the run's first step is recognised on the device.  cont: the step enqueued
+// just before was this run's last with advance set, so nQ = Q already and the
+// step index and CFL are this step's; advance: a step with cont follows.
 int enqueue_step(flow_ctx* c, const flow_params* p, int ts, int hist_slot, int first,
-                 bool device_ts = false) {
+                 bool device_ts = false, bool cont = false, bool advance = false) {
   int rc = 0;
   int total = c->nn + c->ng;
   c->citer = ts;
   if (device_ts) first = -1;
   StepArgs a = make_args(p, ts);
+  a.zero_iterate = 1;
   const int clear = begin_flags(c, p, a);
   // the step index and CFL (k_step_args) by the first thread of the step's
   // first kernel
-  k_begin_step<<<grid_blocks(total, 256), 256, 0, c->stream>>>(
-      c->m, c->s, kBeginCopyQ | kBeginStepArgs | clear, device_ts ? 0 : ts, p->method, p->ramp,
-      p->CFL);
-  rc |= launch_check(c);
+  if (!cont || clear) {
+    k_begin_step<<<grid_blocks(total, 256), 256, 0, c->stream>>>(
+        c->m, c->s, (cont ? 0 : kBeginCopyQ | kBeginStepArgs) | clear, device_ts ? 0 : ts,
+        p->method, p->ramp, p->CFL);
+    rc |= launch_check(c);
+  }
   for (int mi = 1; mi <= p->iter; mi++) {
     int jac = ((mi - 1) % p->jufreq == 0) || mi == 1;
-    if (mi > 1) {
+    if (mi > 1 && clear) {
       // phi <- 1 at every Newton iteration (solve.C:344-348)
       k_begin_step<<<grid_blocks(total, 256), 256, 0, c->stream>>>(c->m, c->s, clear);
       rc |= launch_check(c);
@@ -757,12 +756,14 @@ int enqueue_step(flow_ctx* c, const flow_params* p, int ts, int hist_slot, int f
     rc |= launch_residuals(c, a, jac);
     flow_params pe = *p;  // the sweep schedule may lower the sweep count early on
     pe.subits = sweeps_at(c, p, ts);
-    rc |= launch_linear_solve(c, &pe, false);
+    rc |= launch_linear_solve(c, &pe, false, true);
     const bool last = mi == p->iter;
-    k_finish_step<<<kRedBlocks, kRedThreads, 0, c->stream>>>(
+    k_finish_step<<<std::min(kRedBlocks, grid_blocks(total, kRedThreads)), kRedThreads, 0,
+                    c->stream>>>(
         c->m, c->s, last, last && hist_slot >= 0 ? c->d_hist : nullptr,
         last && hist_slot >= 0 ? c->d_hist + c->hist_cap : nullptr, hist_slot < 0 ? 0 : hist_slot,
-        last ? (first < 0 ? -1 : first) : 0);
+        last ? (first < 0 ? -1 : first) : 0, last && advance,
+        RampArgs{p->method, p->ramp, p->CFL});
     rc |= launch_check(c);
   }
   return rc;
@@ -801,7 +802,7 @@ int enqueue_chunk(flow_ctx* c, const flow_params* p, int ts0, int K) {
                           (c->precision == 0 && (c->sweep_mode == 1 || c->levels.nlev > 0)) ||
                           p->subits % 2 == 0);
   if (!graphable) {
-    for (int i = 0; i < K && !rc; i++) rc |= enqueue_step(c, p, ts0 + i, -1, -1, true);
+    for (int i = 0; i < K && !rc; i++) rc |= enqueue_step(c, p, ts0 + i, -1, -1, true, i > 0, i + 1 < K);
     return rc;
   }
   flow_ctx::ChunkGraph* g = nullptr;
@@ -826,7 +827,7 @@ int enqueue_chunk(flow_ctx* c, const flow_params* p, int ts0, int K) {
       std::shared_lock<std::shared_mutex> gate(g_device_gate);
       e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
       if (e == cudaSuccess) {
-        for (int i = 0; i < K; i++) rc |= enqueue_step(c, p, ts0 + i, -1, -1, true);
+        for (int i = 0; i < K; i++) rc |= enqueue_step(c, p, ts0 + i, -1, -1, true, i > 0, i + 1 < K);
         e = cudaStreamEndCapture(c->stream, &graph);
       }
     }
@@ -856,7 +857,7 @@ int enqueue_chunk(flow_ctx* c, const flow_params* p, int ts0, int K) {
         return FLOW_ERR_CUDA;
       }
       rc = 0;
-      for (int i = 0; i < K && !rc; i++) rc |= enqueue_step(c, p, ts0 + i, -1, -1, true);
+      for (int i = 0; i < K && !rc; i++) rc |= enqueue_step(c, p, ts0 + i, -1, -1, true, i > 0, i + 1 < K);
       return rc;
     }
     ng.launches = c->launches - l0;
@@ -2106,7 +2107,8 @@ int flow_run(flow_ctx* c, const flow_params* p, int ts0, int nsteps, double* r_h
   if ((rc = ensure_hist(c, std::max(nsteps, 1)))) return rc;
   cudaEventRecord(c->ev0, c->stream);
   reset_run(c, 0.);
-  for (int i = 0; i < nsteps && !rc; i++) rc |= enqueue_step(c, p, ts0 + i, i, i == 0);
+  for (int i = 0; i < nsteps && !rc; i++)
+    rc |= enqueue_step(c, p, ts0 + i, i, i == 0, false, i > 0, i + 1 < nsteps);
   cudaEventRecord(c->ev1, c->stream);
   if (rc) return rc;
   int st = read_status(c);
@@ -2134,7 +2136,7 @@ int flow_converge(flow_ctx* c, const flow_params* p, int ts0, int max_steps, dou
     int n = std::min(chunk, max_steps - issued);
     if (issued == 0 || n < chunk) {
       for (int i = 0; i < n && !rc; i++, issued++)
-        rc |= enqueue_step(c, p, ts0 + issued, -1, issued == 0);
+        rc |= enqueue_step(c, p, ts0 + issued, -1, issued == 0, false, i > 0, i + 1 < n);
     } else {
       rc |= enqueue_chunk(c, p, ts0 + issued, n);
       issued += n;
@@ -2211,7 +2213,7 @@ int flow_converge_batch(flow_ctx** ctxs, int n, const flow_params* p, int ts0, i
       int rc = 0;
       if (issued[i] == 0 || k < chunk) {
         for (int q = 0; q < k && !rc; q++, issued[i]++)
-          rc |= enqueue_step(c, p, ts0 + issued[i], -1, issued[i] == 0);
+          rc |= enqueue_step(c, p, ts0 + issued[i], -1, issued[i] == 0, false, q > 0, q + 1 < k);
       } else {
         rc |= enqueue_chunk(c, p, ts0 + issued[i], k);
         issued[i] += k;
@@ -2310,7 +2312,7 @@ int flow_linear_solve(flow_ctx* c, const flow_params* p, double* rms) {
   if (rc) return rc;
   cudaSetDevice(c->device);
   reset_run(c, 0.);
-  rc = launch_linear_solve(c, p, true);
+  rc = launch_linear_solve(c, p, true, false);
   if (rc) return rc;
   int st = read_status(c);
   if (rms) {
@@ -2332,11 +2334,11 @@ int flow_selftest_sweep_timeout(flow_ctx* c, long max_spin, int* status) {
   reset_run(c, 0.);
   cudaMemsetAsync(c->s.status, 0, sizeof(int), c->stream);
   cudaMemsetAsync(c->s.skip, 0, sizeof(int), c->stream);
-  cudaMemcpyAsync(c->s.counter, &kFirst, sizeof(unsigned), cudaMemcpyHostToDevice, c->stream);
   double* dq_new = c->s.dQ2;
   k_prepare_sweep<<<grid_blocks(4 * (c->nn + 1), 256), 256, 0, c->stream>>>(
       c->s, c->s.dQ, dq_new, 4 * (c->nn + 1));
   int rc = launch_check(c);
+  cudaMemcpyAsync(c->s.counter, &kFirst, sizeof(unsigned), cudaMemcpyHostToDevice, c->stream);
   k_sweep_ordered<true><<<c->nsm * 4, 128, 0, c->stream>>>(c->m, c->s, c->s.dQ, dq_new, max_spin);
   rc |= launch_check(c);
   if (rc) return rc;
@@ -2508,11 +2510,11 @@ int flow_residual_stage(flow_ctx* c, const flow_params* p, int jupdate, int ts, 
       const int nbs = grid_blocks(c->ns, 128);
       launch_flux_variant(c->var[1], [&](auto V) {
         if (a.recon == 1) {
-          if (jupdate) k_subedge_flux<1, true, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a);
-          else k_subedge_flux<1, false, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a);
+          if (jupdate) k_subedge_flux<1, true, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, 0);
+          else k_subedge_flux<1, false, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, 0);
         } else {
-          if (jupdate) k_subedge_flux<0, true, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a);
-          else k_subedge_flux<0, false, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a);
+          if (jupdate) k_subedge_flux<0, true, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, 0);
+          else k_subedge_flux<0, false, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, 0);
         }
       });
       rc |= launch_check(c);
@@ -3017,7 +3019,8 @@ int enqueue_steps(flow_ctx* c, const flow_params* p, int ts0, int K) {
   cudaSetDevice(c->device);
   if (ts0 == 1) {
     int rc = 0;
-    for (int i = 0; i < K && !rc; i++) rc |= enqueue_step(c, p, ts0 + i, -1, i == 0);
+    for (int i = 0; i < K && !rc; i++)
+      rc |= enqueue_step(c, p, ts0 + i, -1, i == 0, false, i > 0, i + 1 < K);
     return rc;
   }
   return enqueue_chunk(c, p, ts0, K);

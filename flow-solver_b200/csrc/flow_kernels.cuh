@@ -5,13 +5,17 @@
 //   k_begin_step      step index and CFL, nQ <- Q, and what the node kernel
 //                     will not overwrite of grad/hess <- 0, phi <- 1
 //                                                               (init_memory.C:200-224,
-//                                                                solve.C:298-348)
+//                                                                solve.C:298-348);
+//                     a step that follows another of the same call has nQ = Q
+//                     and its index and CFL from k_finish_step, and needs none
+//                     of it when there is nothing to clear
 //   k_node_prepare    per node: wave-speed sum, dt and V/dt    (build_matrix)
 //                     + LSQ gradient or k=2 derivatives + Venkatakrishnan phi
 //   k_subedge_flux    per subedge: reconstructed Roe flux and the 8-flux
-//                     forward-difference Jacobian               (residual.C, jacobian.C)
-//   k_boundary        per boundary edge: ghost state, boundary flux and
-//                     approximate Jacobian                      (cvbc.C, residual.C)
+//                     forward-difference Jacobian               (residual.C, jacobian.C);
+//                     per boundary edge, in the launch's first blocks: ghost
+//                     state, boundary flux and approximate Jacobian
+//                                                               (cvbc.C, residual.C)
 //   k_assemble        per node: R, RHS, the node's LHS row, LU of the diagonal
 //   k_sweep_ordered   block Gauss-Seidel sweeps in reference row order
 //   k_lin_residual    b - Ax RMS after a sweep                  (linear_algebra.C:348-387)
@@ -52,13 +56,20 @@ struct StepArgs {
   int jac;                  // Jacobian update
   int steady_diag;          // V/dt diagonal (steady runs)
   int skip_bnd;             // assembly of the interior faces only (build_interior_residuals)
+  int zero_iterate;         // the assembly clears the linear solve's iterate (and skip flag)
+};
+
+// The CFL ramp of the steps a run advances through on the device.
+struct RampArgs {
+  int method, ramp;
+  double CFL;
 };
 
 // ---------------------------------------------------------------------------
 // Step index and CFL of the step about to run (init_memory.C:200-216).
 // citer > 0 sets the index; citer == 0 takes the one after the previous step,
 // which lets a captured sequence of steps replay with an advancing ramp.
-__device__ __forceinline__ void step_args_body(DevState& s, int citer, int method, int ramp,
+__device__ __forceinline__ void step_args_body(const DevState& s, int citer, int method, int ramp,
                                                double CFL) {
   const int ci = citer > 0 ? citer : *s.citer + 1;
   *s.citer = ci;
@@ -979,6 +990,11 @@ __device__ __forceinline__ void assemble_row(const DevMesh& m, const DevState& s
   }
   s.R[4 * (long)n + q] = r;
   s.RHS[4 * (long)n + q] = -(r);
+  if (a.zero_iterate) {  // the linear solve starts from zero (linear_algebra.C:165-170)
+    if (MIXED) mt.dq32[4 * (long)n + q] = 0.f;
+    else s.dQ[4 * (long)n + q] = 0.;
+    if (n == 1 && q == 0) *s.skip = 0;
+  }
   const int k0 = m.ia[n], k1 = m.ia[n + 1];
   // precision form: this row's off-diagonal blocks in colour order (the
   // diagonal block is the row's last, so block k is off-diagonal k - k0)
@@ -1243,10 +1259,27 @@ __global__ void __launch_bounds__(128) k_diag_lu(DevMesh m, DevState s) {
 // only): the approximate Roe Jacobian dF/dqL = (A(qL) + |A~|) len / 2,
 // dF/dqR = (A(qR) - |A~|) len / 2 (|A~| frozen: the form jacobian.C:681-962
 // gives the boundary faces), from the |A~| the flux formed anyway.
+// bnd: the launch's first blocks take the boundary edges (boundary_edge), the
+// rest the subedges: the two do not touch one another's data, and the boundary
+// edges' few long chains (9 us by themselves) run beside the faces'.
+template <bool JAC>
+__device__ void boundary_edge(const DevMesh& m, const DevState& s, const StepArgs& a, int b);
+
 template <int RECON, bool JAC, int MINB, int JMODE = 0>
-__global__ void __launch_bounds__(128, MINB) k_subedge_flux(DevMesh m, DevState s, StepArgs a) {
+__global__ void __launch_bounds__(128, MINB) k_subedge_flux(DevMesh m, DevState s, StepArgs a,
+                                                            int bnd) {
   if (*s.stop) return;  // the run has converged
-  int sub = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  int block = blockIdx.x;
+  if (bnd) {
+    const int nb = (m.nbe + 127) / 128;
+    if (block < nb) {
+      const int b = block * 128 + threadIdx.x + 1;
+      if (b <= m.nbe) boundary_edge<JAC>(m, s, a, b);
+      return;
+    }
+    block -= nb;
+  }
+  int sub = block * 128 + threadIdx.x + 1;
   if (sub > m.ns) return;
   const int2 lr = m.sub_lr[sub];
   const double4 g = m.sub_geo[sub];
@@ -1331,10 +1364,7 @@ __global__ void __launch_bounds__(128, MINB) k_subedge_flux(DevMesh m, DevState 
 // the node normal and the arc length and writes the normal back into
 // xn_bedges (residual.C:1103-1143), as the reference does.
 template <bool JAC>
-__global__ void __launch_bounds__(128) k_boundary(DevMesh m, DevState s, StepArgs a) {
-  if (*s.stop) return;  // the run has converged
-  int b = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  if (b > m.nbe) return;
+__device__ void boundary_edge(const DevMesh& m, const DevState& s, const StepArgs& a, int b) {
   int4 info = m.bed_info[b];
   const int rn = info.x, gn = info.y, bc = info.z;
   double* xnb = s.xn_bedges + 3 * (long)b;
@@ -1427,6 +1457,13 @@ __global__ void __launch_bounds__(128) k_boundary(DevMesh m, DevState s, StepArg
   double* Jo = s.Jb + 16 * (long)b;
 #pragma unroll
   for (int k = 0; k < 16; k++) Jo[k] = 0.5 * (d[k] + Rm[k]) * len;
+}
+
+template <bool JAC>
+__global__ void __launch_bounds__(128) k_boundary(DevMesh m, DevState s, StepArgs a) {
+  if (*s.stop) return;  // the run has converged
+  const int b = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  if (b <= m.nbe) boundary_edge<JAC>(m, s, a, b);
 }
 
 // LHS = 0 with V/dt on the diagonal blocks (init_memory.C:189-290).
@@ -1805,6 +1842,7 @@ __global__ void __launch_bounds__(128) k_sweep_ordered32(DevState s, MixedTables
 // (or the current iterate when the sweep will not run).
 __global__ void k_prepare_sweep32(DevState s, const float* cur, float* next, int n) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *s.counter = 0u;  // the sweep's row dispenser
   if (i < 4 || i >= n) return;  // row 0 is unused
   if (*s.stop || *s.skip)
     next[i] = cur[i];
@@ -2406,6 +2444,7 @@ __global__ void __launch_bounds__(kLevelThreads, 1) k_sweep_levels(DevMesh m, De
 // current dQ over instead, so that the buffer swap after the sweep keeps it.
 __global__ void k_prepare_sweep(DevState s, const double* cur, double* next, int n) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *s.counter = 0u;  // the sweep's row dispenser
   if (i < 4 || i >= n) return;  // row 0 is unused (and stays zero)
   if (*s.stop || *s.skip)
     next[i] = cur[i];
@@ -2414,19 +2453,43 @@ __global__ void k_prepare_sweep(DevState s, const double* cur, double* next, int
 }
 
 // ---------------------------------------------------------------------------
-// Deterministic block reduction helper: fixed tree over kRedThreads lanes.
-__device__ __forceinline__ double block_sum(double v, double* sh) {
+// Deterministic block reduction: a fixed tree over kRedThreads lanes (lane i
+// adds lane i + w for w = 128, 64, ... 1), the widths below a warp by
+// exchanges.  N sums at once; every thread gets them.
+template <int N>
+__device__ __forceinline__ void block_sums(double (&v)[N], double* sh) {
+  static_assert(kRedThreads == 256, "the tree's widths");
   const int tid = threadIdx.x;
-  sh[tid] = v;
+#pragma unroll
+  for (int i = 0; i < N; i++) sh[i * kRedThreads + tid] = v[i];
   __syncthreads();
 #pragma unroll
-  for (int w = kRedThreads / 2; w > 0; w >>= 1) {
-    if (tid < w) sh[tid] += sh[tid + w];
+  for (int w = 128; w >= 64; w >>= 1) {
+    if (tid < w)
+#pragma unroll
+      for (int i = 0; i < N; i++) {
+        v[i] += sh[i * kRedThreads + tid + w];
+        sh[i * kRedThreads + tid] = v[i];
+      }
     __syncthreads();
   }
-  double out = sh[0];
+  if (tid < 32)
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      v[i] += sh[i * kRedThreads + tid + 32];
+#pragma unroll
+      for (int w = 16; w > 0; w >>= 1) v[i] += __shfl_down_sync(0xffffffffu, v[i], w);
+      if (tid == 0) sh[i * kRedThreads] = v[i];
+    }
   __syncthreads();
-  return out;
+#pragma unroll
+  for (int i = 0; i < N; i++) v[i] = sh[i * kRedThreads];
+  __syncthreads();
+}
+__device__ __forceinline__ double block_sum(double v, double* sh) {
+  double a[1] = {v};
+  block_sums(a, sh);
+  return a[0];
 }
 
 // |b - Ax|^2 of the rows by quads of lanes, lane q owning component q: row j's
@@ -2556,15 +2619,17 @@ __global__ void __launch_bounds__(kRedThreads) k_lin_residual(DevMesh m, DevStat
 // The step's norms from the per-block partial sums (summed in block order,
 // the same bits whatever block forms them), the history, the run's first
 // residual, the step count and the stop flag.
+// advance: the step index and CFL of the next step too (unless the run stops).
 __device__ __forceinline__ void finalize_step_body(DevState& s, double* sh, double* hist_dq,
-                                                   double* hist_r, int slot, int first) {
-  double a = 0., b = 0.;
-  for (int i = threadIdx.x; i < kRedBlocks; i += blockDim.x) {
-    a += __ldcg(s.partial + i);
-    b += __ldcg(s.partial + kRedBlocks + i);
+                                                   double* hist_r, int slot, int first,
+                                                   int advance, const RampArgs& ra) {
+  double t[2] = {0., 0.};
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
+    t[0] += __ldcg(s.partial + i);
+    t[1] += __ldcg(s.partial + kRedBlocks + i);
   }
-  double ta = block_sum(a, sh);
-  double tb = block_sum(b, sh);
+  block_sums(t, sh);
+  const double ta = t[0], tb = t[1];
   if (threadIdx.x == 0) {
     s.scalars[1] = ta;
     s.scalars[2] = tb;
@@ -2576,6 +2641,7 @@ __device__ __forceinline__ void finalize_step_body(DevState& s, double* sh, doub
     *s.steps_done += 1;
     // stop once ||R_rho|| < drop * ||R_rho|| of the first step
     if (s.scalars[7] > 0. && r < s.scalars[7] * s.scalars[6]) *s.stop = 1;
+    else if (advance) step_args_body(s, 0, ra.method, ra.ramp, ra.CFL);
   }
 }
 
@@ -2586,9 +2652,10 @@ __device__ __forceinline__ void finalize_step_body(DevState& s, double* sh, doub
 // last block sets back to zero.
 __global__ void __launch_bounds__(kRedThreads) k_finish_step(DevMesh m, DevState s, int last,
                                                             double* hist_dq, double* hist_r,
-                                                            int slot, int first) {
+                                                            int slot, int first, int advance,
+                                                            RampArgs ra) {
   if (*s.stop) return;  // the run has converged (every block sees the same flag)
-  __shared__ double sh[kRedThreads];
+  __shared__ double sh[2 * kRedThreads];
   __shared__ int is_last;
   double dq2 = 0., r2 = 0.;
   const int total = m.nn + m.ng;
@@ -2608,19 +2675,19 @@ __global__ void __launch_bounds__(kRedThreads) k_finish_step(DevMesh m, DevState
       reinterpret_cast<double4*>(s.Q)[i] = nq;
     }
   }
-  double a = block_sum(dq2, sh);
-  double b = block_sum(r2, sh);
+  double t[2] = {dq2, r2};
+  block_sums(t, sh);
   unsigned* done = reinterpret_cast<unsigned*>(s.partial + 2 * kRedBlocks);
   if (threadIdx.x == 0) {
-    s.partial[blockIdx.x] = a;
-    s.partial[kRedBlocks + blockIdx.x] = b;
+    s.partial[blockIdx.x] = t[0];
+    s.partial[kRedBlocks + blockIdx.x] = t[1];
     __threadfence();  // the partials are visible before the count says so
     is_last = atomicAdd(done, 1u) == gridDim.x - 1;
   }
   __syncthreads();
   if (!is_last) return;
   __threadfence();
-  finalize_step_body(s, sh, hist_dq, hist_r, slot, first);
+  finalize_step_body(s, sh, hist_dq, hist_r, slot, first, advance, ra);
   if (threadIdx.x == 0) *done = 0u;
 }
 
