@@ -287,6 +287,24 @@ int launch_check(flow_ctx* c) {
   return 0;
 }
 
+// Launch k, whose kernel waits for the one before it on the stream by itself
+// (after_wait in flow_kernels.cuh): its blocks start as soon as that one's have
+// all triggered.  Behind anything but a kernel that triggers it starts as usual.
+template <class... P, class... A>
+void launch_after(flow_ctx* c, void (*k)(P...), int grid, int threads, size_t smem, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
+}
+
 StepArgs make_args(const flow_params* p, int ts) {
   StepArgs a{};
   a.gamma = p->gamma;
@@ -518,7 +536,7 @@ int launch_residuals(flow_ctx* c, const StepArgs& a, int jac) {
 
 // The mode 3 sweep kernels by lanes a row, CTA shape and direction: one
 // colour, a colour's two passes in a row, a whole sweep in one launch.
-using ChunkKernel = void (*)(DevState, ChunkTables, float*, int, int);
+using ChunkKernel = void (*)(DevState, ChunkTables, float*, int, int, int);
 using ChunkDfKernel = void (*)(DevState, ChunkTables, float*, int, long);
 template <int L>
 struct ChunkKernels {
@@ -548,6 +566,7 @@ ChunkDfKernel chunk_df_kernel(const ChunkTables& ct, int dir) {
 // cleared: the assembly before this left the iterate zero (StepArgs::zero_iterate).
 int launch_linear_solve_mixed(flow_ctx* c, const flow_params* p, bool cleared) {
   int rc = 0;
+  int first = 1;  // the sweep launch behind the assembly, which writes the matrix
   // the last sweep writes every row of the FP64 dQ
   if (!cleared || p->subits < 1)
     cudaMemsetAsync(c->s.dQ, 0, sizeof(double) * 4 * (c->nn + 1), c->stream);
@@ -572,8 +591,9 @@ int launch_linear_solve_mixed(flow_ctx* c, const flow_params* p, bool cleared) {
         const int last = (pair ? passes[k + 1].first : it) == p->subits - 1;
         if (pair) k++;
         if (nb <= 0) continue;
-        chunk_kernel(ct, dir, pair)<<<nb, threads, smem, c->stream>>>(c->s, ct, c->mt.dq32, col,
-                                                                     last);
+        launch_after(c, chunk_kernel(ct, dir, pair), nb, threads, smem, c->s, ct, c->mt.dq32, col,
+                     last, first);
+        first = 0;
         rc |= launch_check(c);
       }
       return rc;
@@ -593,8 +613,9 @@ int launch_linear_solve_mixed(flow_ctx* c, const flow_params* p, bool cleared) {
         const int col = dir == 0 ? ci : ct.ncol - 1 - ci;
         const int nb = c->h_col_ptr[col + 1] - c->h_col_ptr[col];
         if (nb <= 0) continue;
-        chunk_kernel(ct, dir, false)<<<nb, threads, smem, c->stream>>>(c->s, ct, c->mt.dq32, col,
-                                                                      last);
+        launch_after(c, chunk_kernel(ct, dir, false), nb, threads, smem, c->s, ct, c->mt.dq32, col,
+                     last, first);
+        first = 0;
         rc |= launch_check(c);
       }
     }
@@ -631,8 +652,9 @@ int launch_linear_solve_mixed(flow_ctx* c, const flow_params* p, bool cleared) {
       const int p0 = c->h_color_ptr[col], p1 = c->h_color_ptr[col + 1];
       const int nb = grid_blocks(4 * (p1 - p0), 128);
       if (nb == 0) continue;
-      if (last) k_sweep_color32<true><<<nb, 128, 0, c->stream>>>(c->s, c->mt, p0, p1);
-      else k_sweep_color32<false><<<nb, 128, 0, c->stream>>>(c->s, c->mt, p0, p1);
+      launch_after(c, last ? k_sweep_color32<true> : k_sweep_color32<false>, nb, 128, 0, c->s,
+                   c->mt, p0, p1, first);
+      first = 0;
       rc |= launch_check(c);
     }
   }
