@@ -184,7 +184,7 @@ struct flow_ctx {
   // one-CTA ordered sweep: stage tables (null when the matrix bandwidth is too
   // large for its dQ window, then the multi-CTA sweep is used)
   SweepTables sweep_tb{};
-  LevelTables levels{};  // FP64 sweep by levels (build_levels); nlev 0: not used
+  BandTables bands{};    // FP64 sweep by bands (build_bands); nband 0: not used
   bool sweep_cta_ok = false;
   double* d_hist = nullptr;  // 2 x hist_cap device history of (dq, r_rho)
   int hist_cap = 0;
@@ -396,7 +396,7 @@ void harvest(flow_ctx* c) {
 // chains split over 16 lanes).
 constexpr int kVariants = 3;
 constexpr int kNodeVariants = 8;
-constexpr int kLevelSmemMax = 227 * 1024;  // k_sweep_levels
+constexpr int kLevelSmemMax = 226 * 1024;  // k_sweep_bands
 constexpr size_t kStageSmemMax = 110 * 1024;  // two CTAs per SM at most
 using NodeKernel = void (*)(DevMesh, DevState, StepArgs);
 struct NodeForm {
@@ -679,13 +679,6 @@ int launch_linear_solve(flow_ctx* c, const flow_params* p, bool final_rms, bool 
         else
           k_sweep_cta<false><<<1, kSweepThreads, sm, c->stream>>>(c->m, c->s, c->sweep_tb, max_spin);
         rc |= launch_check(c);
-      } else if (c->levels.nlev > 0) {
-        const size_t sm = level_smem_bytes(c->levels.nlev, c->levels.ring);
-        if (it % 2 == 0)
-          k_sweep_levels<true><<<1, kLevelThreads, sm, c->stream>>>(c->m, c->s, c->levels, it == 0);
-        else
-          k_sweep_levels<false><<<1, kLevelThreads, sm, c->stream>>>(c->m, c->s, c->levels, 0);
-        rc |= launch_check(c);
       } else {
         // results go to the other dQ buffer, pre-filled with the not-ready
         // pattern; the buffers swap roles afterwards
@@ -693,8 +686,16 @@ int launch_linear_solve(flow_ctx* c, const flow_params* p, bool final_rms, bool 
         k_prepare_sweep<<<grid_blocks(4 * (c->nn + 1), 256), 256, 0, c->stream>>>(
             c->s, c->s.dQ, dq_new, 4 * (c->nn + 1));
         rc |= launch_check(c);
-        int blocks = c->nsm * 4;
-        if (it % 2 == 0)
+        const int blocks = c->nsm * 4;
+        const BandTables& bt = c->bands;
+        const size_t sm = band_smem_bytes(bt.levels, bt.places);
+        if (bt.nband > 0 && it % 2 == 0)
+          k_sweep_bands<true><<<bt.nband, kLevelThreads, sm, c->stream>>>(c->s, bt, c->s.dQ, dq_new,
+                                                                         max_spin);
+        else if (bt.nband > 0)
+          k_sweep_bands<false><<<bt.nband, kLevelThreads, sm, c->stream>>>(c->s, bt, c->s.dQ, dq_new,
+                                                                          max_spin);
+        else if (it % 2 == 0)
           k_sweep_ordered<true><<<blocks, 128, 0, c->stream>>>(c->m, c->s, c->s.dQ, dq_new, max_spin);
         else
           k_sweep_ordered<false><<<blocks, 128, 0, c->stream>>>(c->m, c->s, c->s.dQ, dq_new, max_spin);
@@ -821,7 +822,7 @@ int enqueue_chunk(flow_ctx* c, const flow_params* p, int ts0, int K) {
   const bool graphable = c->use_graphs && !c->timing && K > 0 && ph == phase_of(p, ts0 + K - 1) &&
                          sw == sweeps_at(c, p, ts0 + K - 1) &&
                          (c->precision == 1 || c->precision == 3 ||
-                          (c->precision == 0 && (c->sweep_mode == 1 || c->levels.nlev > 0)) ||
+                          (c->precision == 0 && c->sweep_mode == 1) ||
                           p->subits % 2 == 0);
   if (!graphable) {
     for (int i = 0; i < K && !rc; i++) rc |= enqueue_step(c, p, ts0 + i, -1, -1, true, i > 0, i + 1 < K);
@@ -1069,7 +1070,7 @@ bool ensure_kernel_attrs(int device) {
                         (const void*)k_faces_assemble<0, 2>, (const void*)k_faces_assemble<1, 2>})
     ok = ok && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)kFusedSmem) == cudaSuccess;
-  for (const void* f : {(const void*)k_sweep_levels<true>, (const void*)k_sweep_levels<false>})
+  for (const void* f : {(const void*)k_sweep_bands<true>, (const void*)k_sweep_bands<false>})
     ok = ok && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kLevelSmemMax) ==
                    cudaSuccess;
   for (const void* f : {(const void*)k_sweep_cta<true>, (const void*)k_sweep_cta<false>})
@@ -1079,12 +1080,12 @@ bool ensure_kernel_attrs(int device) {
   return ok;
 }
 
-// Tables of k_sweep_levels, where the matrix suits it: at most kRecBlocks
-// off-diagonal blocks a row with the diagonal block last, levels that are not
-// too wide, and a window of dQ that fits in shared memory.  Otherwise, and
-// where the tables find no room, the context keeps the grid-wide sweep.
-void build_levels(flow_ctx* c) {
-  if (c->levels.nlev > 0) return;
+// Tables of k_sweep_bands, where the matrix suits it: at most kRecBlocks
+// off-diagonal blocks a row with the diagonal block last, and bands whose rows
+// and halo fit in shared memory.  Otherwise, and where the tables find no room,
+// the context keeps the grid-wide sweep.
+void build_bands(flow_ctx* c) {
+  if (c->bands.nband > 0) return;
   const int nn = c->nn;
   const std::vector<int>& ia = c->h_ia;
   const std::vector<int>& ja = c->h_ja;
@@ -1099,97 +1100,110 @@ void build_levels(flow_ctx* c) {
     lev[j] = l;
     nlev = std::max(nlev, l + 1);
   }
-  if (nlev > kLevelMax || nn > (long)kLevelWidthMax * nlev) return;
-  // tiles and positions: level by level, rows ascending
-  std::vector<int> count(nlev + 1, 0), lev_tile(nlev + 1, 0), pos(nn + 1, 0);
-  for (int j = 1; j <= nn; j++) count[lev[j] + 1]++;
-  for (int l = 0; l < nlev; l++) {
-    lev_tile[l + 1] = lev_tile[l] + (count[l + 1] + 7) / 8;
-    count[l + 1] += count[l];
-  }
-  {
-    std::vector<int> at(count.begin(), count.end() - 1);
-    for (int j = 1; j <= nn; j++) pos[j] = at[lev[j]]++;
-  }
-  // positions a level touches (its rows and their columns)
-  std::vector<int> first(nlev, nn), last(nlev, -1);
-  for (int j = 1; j <= nn; j++) {
-    int lo = nn, hi = -1;
-    for (int k = ia[j]; k < ia[j + 1]; k++) {
-      lo = std::min(lo, pos[ja[k]]);
-      hi = std::max(hi, pos[ja[k]]);
+  // both directions run by these levels: a row's upper neighbours lie above it
+  for (int j = 1; j <= nn; j++)
+    for (int k = ia[j]; k < ia[j + 1] - 1; k++)
+      if (ja[k] > j && lev[ja[k]] <= lev[j]) return;
+  const int per = kBandRows, nband = (nn + per - 1) / per;
+  // rows by level, ascending inside a level
+  std::vector<int> first(nlev + 1, 0), order(nn);
+  for (int j = 1; j <= nn; j++) first[lev[j] + 1]++;
+  for (int l = 0; l < nlev; l++) first[l + 1] += first[l];
+  for (int j = 1; j <= nn; j++) order[first[lev[j]]++] = j;
+  // the same per band (bands have `per` rows but the last)
+  std::vector<int> fill(nband), rows(nn);
+  for (int b = 0; b < nband; b++) fill[b] = b * per;
+  for (int j : order) rows[fill[(j - 1) / per]++] = j;
+  std::vector<Band> bands(nband);
+  std::vector<LevelSlot> slots;
+  std::vector<int2> levs, halo;
+  slots.reserve(2 * (size_t)nn);
+  std::vector<int> place(nn + 1, 0), seen(nn + 1, -1), local(per);
+  BandTables bt{};
+  for (int b = 0; b < nband; b++) {
+    Band& B = bands[b];
+    B.row0 = b * per + 1;
+    B.nrows = std::min(per, nn - b * per);
+    const int* R = rows.data() + b * per;
+    const int end = B.row0 + B.nrows;
+    B.lev0 = (int)levs.size();
+    B.halo0 = (int)halo.size();
+    for (int i = 0; i < B.nrows; i++)
+      local[i] = i == 0 ? 0 : local[i - 1] + (lev[R[i]] != lev[R[i - 1]]);
+    B.nlev = local[B.nrows - 1] + 1;
+    levs.resize(B.lev0 + B.nlev, make_int2(0, 0));
+    // rows before the band in the order in which the levels need them forward,
+    // rows behind it in the order backward
+    for (int i = 0; i < B.nrows; i++)
+      for (int k = ia[R[i]]; k < ia[R[i] + 1]; k++)
+        if (ja[k] < B.row0 && seen[ja[k]] != b) {
+          seen[ja[k]] = b;
+          place[ja[k]] = B.nrows + B.nlo++;
+          halo.push_back(make_int2(ja[k], place[ja[k]] | local[i] << 16));
+          levs[B.lev0 + local[i]].y++;
+        }
+    for (int i = B.nrows - 1; i >= 0; i--)
+      for (int k = ia[R[i]]; k < ia[R[i] + 1]; k++)
+        if (ja[k] >= end && seen[ja[k]] != b) {
+          seen[ja[k]] = b;
+          place[ja[k]] = B.nrows + B.nlo + B.nhi++;
+          halo.push_back(make_int2(ja[k], place[ja[k]] | local[i] << 16));
+          levs[B.lev0 + local[i]].y += 1 << 16;
+        }
+    const int none = B.nrows + B.nlo + B.nhi;
+    if (none >= 32768 || B.nlev >= 32768 || B.nlo >= 32768 || B.nhi >= 32768) return;
+    bt.places = std::max(bt.places, none);
+    bt.levels = std::max(bt.levels, B.nlev);
+    if (band_smem_bytes(bt.levels, bt.places) > (size_t)kLevelSmemMax) return;
+    B.tile0 = (int)(slots.size() / 8);
+    for (int i = 0; i < B.nrows; i++) {
+      const int j = R[i], nb = ia[j + 1] - ia[j] - 1;
+      if (i == 0 || local[i] != local[i - 1]) slots.resize((slots.size() + 7) & ~(size_t)7);
+      if (slots.size() % 8 == 0) levs[B.lev0 + local[i]].x++;
+      LevelSlot S{};
+      S.row = j;
+      S.block = ia[j];
+      S.level_nb = (unsigned)local[i] | (unsigned)nb << 28;
+      S.pos = j - B.row0;
+      unsigned q[kRecBlocks];
+      for (int t = 0; t < kRecBlocks; t++) {
+        const int col = t < nb ? ja[ia[j] + t] : 0;
+        q[t] = t >= nb ? none : col >= B.row0 && col < end ? col - B.row0 : place[col];
+      }
+      S.cols = make_uint4(q[0] | q[1] << 16, q[2] | q[3] << 16, q[4] | q[5] << 16,
+                          q[6] | q[7] << 16);
+      slots.push_back(S);
     }
-    first[lev[j]] = std::min(first[lev[j]], lo);
-    last[lev[j]] = std::max(last[lev[j]], hi);
+    slots.resize((slots.size() + 7) & ~(size_t)7);
+    B.ntile = (int)(slots.size() / 8) - B.tile0;
+    // an empty slot reads zeros and belongs to its tile's level
+    for (size_t i = 8 * (size_t)B.tile0; i < slots.size(); i++)
+      if (slots[i].row == 0) {
+        slots[i].cols = make_uint4(none * 65537u, none * 65537u, none * 65537u, none * 65537u);
+        slots[i].level_nb = slots[i - i % 8].level_nb & 0xfffffff;
+      }
   }
-  // per direction (its levels in running order): the positions that must be in
-  // the window before each level, and the smallest ring in which none is
-  // overwritten before the levels that read the old one are done
-  std::vector<int> to[2] = {std::vector<int>(nlev), std::vector<int>(nlev)};
-  int ring = 1;
-  for (int dir = 0; dir < 2; dir++) {
-    std::vector<int> back(nlev);  // the farthest position that level o or a later one touches
-    for (int o = 0; o < nlev; o++) {
-      const int l = dir == 0 ? o : nlev - 1 - o;
-      to[dir][o] = dir == 0 ? std::max(o > 0 ? to[0][o - 1] : 0, last[l] + 1)
-                            : std::min(o > 0 ? to[1][o - 1] : nn, first[l]);
-    }
-    for (int o = nlev - 1; o >= 0; o--) {
-      const int l = dir == 0 ? o : nlev - 1 - o;
-      back[o] = dir == 0 ? first[l] : last[l];
-      if (o + 1 < nlev)
-        back[o] = dir == 0 ? std::min(back[o], back[o + 1]) : std::max(back[o], back[o + 1]);
-    }
-    // while the rows for level o are loaded, levels from o - kLevelsAhead on may run
-    for (int o = 0; o < nlev; o++) {
-      const int b = back[std::max(0, o - kLevelsAhead)];
-      ring = std::max(ring, dir == 0 ? to[0][o] - b : b - to[1][o] + 1);
-    }
-  }
-  if (ring >= 65535 || level_smem_bytes(nlev, ring) > (size_t)kLevelSmemMax) return;
-  std::vector<LevelSlot> slots(8 * (size_t)lev_tile[nlev]);
-  LevelSlot empty{};
-  empty.cols = make_uint4(ring * 65537u, ring * 65537u, ring * 65537u, ring * 65537u);
-  for (int l = 0; l < nlev; l++) {
-    empty.level_nb = (unsigned)l;
-    std::fill(slots.begin() + 8 * (size_t)lev_tile[l], slots.begin() + 8 * (size_t)lev_tile[l + 1],
-              empty);
-  }
-  for (int j = 1; j <= nn; j++) {
-    const int l = lev[j], nb = ia[j + 1] - ia[j] - 1;
-    LevelSlot& S = slots[8 * (size_t)lev_tile[l] + (pos[j] - count[l])];
-    S.row = j;
-    S.block = ia[j];
-    S.level_nb = (unsigned)l | (unsigned)nb << 28;
-    S.pos = pos[j];
-    unsigned q[kRecBlocks];
-    for (int t = 0; t < kRecBlocks; t++)
-      q[t] = t < nb ? (unsigned)(pos[ja[ia[j] + t]] % ring) : (unsigned)ring;
-    S.cols = make_uint4(q[0] | q[1] << 16, q[2] | q[3] << 16, q[4] | q[5] << 16, q[6] | q[7] << 16);
-  }
-  // one buffer: the slots, then the tiles of each level and the two load lists
-  static_assert(sizeof(LevelSlot) == 2 * sizeof(int4), "LevelSlot layout");
-  const size_t nints = (size_t)(nlev + 1) + 2 * (size_t)nlev;
-  std::vector<LevelSlot> all(slots);
-  all.resize(slots.size() + (4 * nints + sizeof(LevelSlot) - 1) / sizeof(LevelSlot));
-  int* ints = reinterpret_cast<int*>(all.data() + slots.size());
-  std::copy(lev_tile.begin(), lev_tile.end(), ints);
-  std::copy(to[0].begin(), to[0].end(), ints + nlev + 1);
-  std::copy(to[1].begin(), to[1].end(), ints + 2 * nlev + 1);
+  // one buffer: the slots, then the bands, the levels and the halo rows
+  const size_t nslots = slots.size(), nb = bands.size(), nl = levs.size(), nh = halo.size();
+  const size_t bytes = sizeof(Band) * nb + sizeof(int2) * (nl + nh) + 8;
+  slots.resize(nslots + (bytes + sizeof(LevelSlot) - 1) / sizeof(LevelSlot));
+  char* tail = reinterpret_cast<char*>(slots.data() + nslots);
+  int2* at = reinterpret_cast<int2*>(tail);
+  std::copy(levs.begin(), levs.end(), at);
+  std::copy(halo.begin(), halo.end(), at + nl);
+  std::copy(bands.begin(), bands.end(), reinterpret_cast<Band*>(at + nl + nh));
   const bool was = c->buf.carve_failed;
-  const LevelSlot* d = upload_vec(c, all);
+  const LevelSlot* d = upload_vec(c, slots);
   if (!d) {  // no room: the grid-wide sweep
     c->buf.carve_failed = was;
     return;
   }
-  LevelTables lt{};
-  lt.ring = ring;
-  lt.slots = d;
-  lt.lev_tile = reinterpret_cast<const int*>(d + slots.size());
-  lt.load_to[0] = lt.lev_tile + nlev + 1;
-  lt.load_to[1] = lt.lev_tile + 2 * nlev + 1;
-  lt.nlev = nlev;
-  c->levels = lt;
+  bt.slots = d;
+  bt.lev = reinterpret_cast<const int2*>(d + nslots);
+  bt.halo = bt.lev + nl;
+  bt.bands = reinterpret_cast<const Band*>(bt.halo + nh);
+  bt.nband = nband;
+  c->bands = bt;
 }
 
 // Mode 3 reads none of the mode 1 / 2 tables: only the FP32 iterate.
@@ -1863,7 +1877,7 @@ static flow_ctx* create_impl(flow_arena* arena, const flow_grid_view* g, const f
     return fail(c, FLOW_ERR_CUDA, "upload failed");
   // an arena's contexts mostly run the precision form: they build the FP64
   // sweep's tables when they are set to precision 0
-  if (!arena) build_levels(c);
+  if (!arena) build_bands(c);
   // the context's own stream only: a device-wide synchronisation here would
   // invalidate a graph capture another thread has open
   if (cudaStreamSynchronize(c->stream) != cudaSuccess)
@@ -1932,10 +1946,10 @@ int flow_set_precision(flow_ctx* c, int mode) {
     int rc = mode == 3 ? build_chunk_iterate(c) : build_mixed_tables(c, mode >= 2);
     if (!rc && mode == 3) rc = build_chunk_tables(c);
     if (rc) return rc;
-  } else if (c->levels.nlev == 0) {
+  } else if (c->bands.nband == 0) {
     cudaStreamSynchronize(c->stream);
     drop_graphs(c);
-    build_levels(c);
+    build_bands(c);
   }
   c->precision = mode;
   return 0;

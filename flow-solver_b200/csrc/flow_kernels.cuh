@@ -1503,8 +1503,7 @@ __global__ void __launch_bounds__(128) k_diag_only(DevMesh m, DevState s) {
 
 // ---------------------------------------------------------------------------
 // Ordered block Gauss-Seidel sweep (linear_algebra.C:178-344) over the whole
-// GPU, for matrices whose levels are wide (kLevelWidthMax; k_sweep_levels
-// otherwise).  Rows are
+// GPU, for matrices that k_sweep_bands does not take (build_bands).  Rows are
 // handed out in the reference's order (ascending forward, descending
 // backward) by an atomic dispenser; one warp per row.  The sweep writes its
 // results into dq_new, which is filled with an all-ones bit pattern (a NaN
@@ -1982,8 +1981,8 @@ __device__ __forceinline__ void level_arrive(unsigned long long* bar) {
 // written in PTX so that its branches are uniform: the caller's exchanges
 // between lanes then need no reconvergence of the warp.
 constexpr int kLevelTries = 1 << 16;
-__device__ __forceinline__ int level_wait(unsigned long long* bar, unsigned parity) {
-  int left = kLevelTries;
+__device__ __forceinline__ int level_wait(unsigned long long* bar, unsigned parity,
+                                          int left = kLevelTries) {
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "LEVEL_TRY:\n\t"
@@ -2290,187 +2289,247 @@ __global__ void __launch_bounds__(32 * ring_warps(0)) k_sweep_chunk_df(DevState 
   }
 }
 
-// The FP64 ordered sweep by one CTA: the rows by dependency level, a tile of
-// 8 rows a warp, four lanes a row (lane r owning block row r), a level handed
-// over by an mbarrier that counts its tiles, as in k_sweep_chunk.  dQ is
-// updated in place, kept both by row (s.dQ) and by position in level order
-// (s.dQ2); the CTA keeps a window of the latter in shared memory (a ring; the
-// place after it holds zeros, which unused blocks read).  One more warp loads
-// the window ahead of the levels (kLevelsAhead) and counts as arrivals of the
-// level two before the one that needs the rows; a place of the ring is
-// overwritten only once every level that reads the old one is done (host-checked,
-// build_levels).  fresh: dQ is zero (the first sweep), nothing is loaded.
-//
-// Bound by the chain of levels: the row-by-row sweep over the whole GPU
-// (k_sweep_ordered) pays a publish and a poll through L2 a level, about 925
-// cycles, besides the row's own chain; inside one SM the hand-over takes 110
-// and a level of one or two tiles 1,150 in all (FP64 latency: reads and
-// products 400, the ordered subtraction 60, the 4x4 solve 500).  Wide levels
-// are bound by the tiles one SM works on at a time, and the whole GPU is the
-// faster one: us a sweep, one CTA against k_sweep_ordered, at 11 rows a level
-// (1,024 rows) 52 / 92, at 19 (4,096) 134 / 196, at 33 (10,816) 273 / 306, at
-// 49 (25,600) 638 / 471.  kLevelWidthMax draws the line.  Forming the
-// products with earlier levels' columns before the wait (two blocks a row
-// reloaded or the tile's waiting blocks formed again after it) measured
-// slower: the registers or branches it takes cost more than the chain gains.
-constexpr int kLevelWidthMax = 34;  // mean rows a level
-constexpr int kLevelWarps = 7;      // tiles in flight (255 registers a thread)
-constexpr int kLevelThreads = 32 * (kLevelWarps + 1);
-constexpr int kLevelsAhead = 3;     // levels the window is loaded ahead
-constexpr int kLevelMax = 8192;     // levels (their barriers sit in shared memory)
+// A lane's share of a row of k_sweep_bands: its slot's words.
+struct LevelRow { int j, block; unsigned ln; int pos; uint4 c; };
 
-__host__ __device__ inline size_t level_smem_bytes(int nlev, int ring) {
-  return 32 * ((size_t)ring + 1) + 8 * (size_t)nlev;
+__device__ __forceinline__ void load_level_row(const LevelSlot* slots, bool in, int tile, int w,
+                                               LevelRow& R) {
+  if (in) {
+    const LevelSlot* S = slots + 8 * (long)tile + w;
+    const int4 q = *reinterpret_cast<const int4*>(S);
+    R.j = q.x;
+    R.block = q.y;
+    R.ln = (unsigned)q.z;
+    R.pos = q.w;
+    R.c = S->cols;
+  }
+}
+// Pins the words in front of the loads that follow (a move behind those would
+// wait for them).
+__device__ __forceinline__ void hold_level_row(LevelRow& h) {
+  asm volatile("" : "+r"(h.j), "+r"(h.block), "+r"(h.ln), "+r"(h.pos)::"memory");
+  asm volatile("" : "+r"(h.c.x), "+r"(h.c.y), "+r"(h.c.z), "+r"(h.c.w)::"memory");
 }
 
-template <bool FWD>
-__global__ void __launch_bounds__(kLevelThreads, 1) k_sweep_levels(DevMesh m, DevState s,
-                                                                  LevelTables lt, int fresh) {
-  if (*s.stop || *s.skip) return;  // converged, or the linear residual dropped below 1e-15
-  extern __shared__ __align__(16) double2 level_smem[];
-  double2* win = level_smem;  // two words a row
-  unsigned long long* bars = reinterpret_cast<unsigned long long*>(win + 2 * (lt.ring + 1));
-  const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31, r = lane & 3, w = lane >> 2;
-  const int warp = __shfl_sync(FULL, (int)threadIdx.x >> 5, 0);  // uniform in the warp
-  const int nlev = lt.nlev;
-  const int ntile = lt.lev_tile[nlev];
-  const int* load_to = lt.load_to[FWD ? 0 : 1];
-  double2* dqp = reinterpret_cast<double2*>(s.dQ2);  // dQ by position, from 1
-  for (int o = threadIdx.x; o < nlev; o += kLevelThreads) {
-    const int l = FWD ? o : nlev - 1 - o;  // the o-th level to run
-    // the level's tiles, and the loader's lanes for the level after the next
-    level_init(bars + o, (unsigned)(lt.lev_tile[l + 1] - lt.lev_tile[l] + (o + 2 < nlev ? 32 : 0)));
-  }
-  // positions p0 .. p1 - 1 into their places of the ring
-  auto load_window = [&](int p0, int p1, int tid, int nt) {
-    for (int i = 2 * p0 + tid; i < 2 * p1; i += nt) {
-      double2* at = win + 2 * ((i >> 1) % lt.ring) + (i & 1);
-      if (fresh) *at = make_double2(0., 0.);
-      else cp_async16(at, dqp + 2 + i);
-    }
-  };
-  if (threadIdx.x < 2) win[2 * lt.ring + threadIdx.x] = make_double2(0., 0.);
-  const int to1 = load_to[min(1, nlev - 1)];  // the first two levels' rows
-  load_window(FWD ? 0 : to1, FWD ? to1 : m.nn, threadIdx.x, kLevelThreads);
-  cp_async_commit();
-  cp_async_wait<0>();
-  bool timeout = false;
-  if (warp == kLevelWarps) {
-    // ---- the loader ----
-    __syncthreads();
-    int from = to1;
-    for (int o = 2; o < nlev; o++) {
-      const int to = load_to[o];
-      if (o > kLevelsAhead) timeout |= !level_wait(bars + o - 1 - kLevelsAhead, 0);
-      if (FWD) load_window(from, to, lane, 32);
-      else load_window(to, from, lane, 32);
-      from = to;
-      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(
-                       static_cast<uint32_t>(__cvta_generic_to_shared(bars + o - 2)))
-                   : "memory");
-    }
-    cp_async_commit();
-    cp_async_wait<0>();
-  } else {
-    auto tile_at = [&](int k) { return FWD ? k : ntile - 1 - k; };
-    struct Row { int j, block; unsigned ln; int pos; uint4 c; };
-    Row h{}, hn{};
-    double4 a[kRecBlocks];
-    double rhs = 0.;
+// A warp's tile of 8 rows, four lanes a row: blocks, right-hand side and, in
+// lane i < 8, the factors of its row i.
+struct LevelTile {
+  double4 a[kRecBlocks], m0, m1, m2, m3, mr;
+  double rhs;
+  __device__ __forceinline__ LevelTile() : rhs(0.) {
     const double4 z4 = make_double4(0., 0., 0., 0.);
 #pragma unroll
     for (int t = 0; t < kRecBlocks; t++) a[t] = z4;
-    double4 m0 = z4, m1 = z4, m2 = z4, m3 = z4, mr = z4;
-    auto load_row = [&](int k, Row& R) {
-      if (k < ntile) {
-        const LevelSlot* S = lt.slots + 8 * (long)tile_at(k) + w;
-        const int4 q = *reinterpret_cast<const int4*>(S);
-        R.j = q.x;
-        R.block = q.y;
-        R.ln = (unsigned)q.z;
-        R.pos = q.w;
-        R.c = S->cols;
-      }
-    };
-    auto load_tile = [&](int k, const Row& R) {
-      if (k < ntile) {
-        const double* A = s.LHS + 16 * (long)R.block + 4 * r;
-        const int nb = R.ln >> 28;
+    m0 = m1 = m2 = m3 = mr = z4;
+  }
+  __device__ __forceinline__ void load(const DevState& s, bool in, const LevelRow& R, int r,
+                                       int lane) {
+    if (in) {
+      const double4 z4 = make_double4(0., 0., 0., 0.);
+      const double* A = s.LHS + 16 * (long)R.block + 4 * r;
+      const int nb = R.ln >> 28;
 #pragma unroll
-        for (int t = 0; t < kRecBlocks; t++) a[t] = t < nb ? ld_d4(A + 16 * t) : z4;
-        rhs = s.RHS[4 * (long)R.j + r];
-        const int j = __shfl_sync(FULL, R.j, 4 * lane);  // row of slot `lane`
-        if (lane < 8) {
-          const double* L = s.LUd + 16 * (long)j;
-          m0 = ld_d4(L);
-          m1 = ld_d4(L + 4);
-          m2 = ld_d4(L + 8);
-          m3 = ld_d4(L + 12);
-          mr = ld_d4(s.LUr + 4 * (long)j);
-        }
-      }
-    };
-    int k = warp;
-    load_row(k, h);
-    load_row(k + kLevelWarps, hn);
-    load_tile(k, h);
-    __syncthreads();
-    for (; k < ntile; k += kLevelWarps) {
-      const int j = __shfl_sync(FULL, h.j, 4 * lane);  // the row lane < 8 solves
-      const int pos = __shfl_sync(FULL, h.pos, 4 * lane);
-      const bool row = j > 0 && lane < 8;
-      const int lev = __shfl_sync(FULL, h.ln & 0xfffffff, 0);
-      const int o = FWD ? lev : nlev - 1 - lev;
-      const double2* d[kRecBlocks] = {
-          win + 2 * (h.c.x & 0xffff), win + 2 * (h.c.x >> 16), win + 2 * (h.c.y & 0xffff),
-          win + 2 * (h.c.y >> 16),    win + 2 * (h.c.z & 0xffff), win + 2 * (h.c.z >> 16),
-          win + 2 * (h.c.w & 0xffff), win + 2 * (h.c.w >> 16)};
-      double2* own = win + 2 * (pos % lt.ring);
-      if (o > 0) timeout |= !level_wait(bars + o - 1, 0);
-      double term[kRecBlocks];
-#pragma unroll
-      for (int t = 0; t < kRecBlocks; t++) {
-        const double2 x01 = d[t][0], x23 = d[t][1];
-        term[t] = (a[t].x * x01.x + a[t].y * x01.y + a[t].z * x23.x + a[t].w * x23.y);
-      }
-      const double2 own01 = own[0], own23 = own[1];
-      // an unused block's term is +0, and acc - 0 is acc, whatever its sign
-      double acc = rhs;
-#pragma unroll
-      for (int t = 0; t < kRecBlocks; t++) acc -= term[t];
-      const double b[4] = {__shfl_sync(FULL, acc, 4 * lane), __shfl_sync(FULL, acc, 4 * lane + 1),
-                           __shfl_sync(FULL, acc, 4 * lane + 2),
-                           __shfl_sync(FULL, acc, 4 * lane + 3)};
-      const double M[16] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w,
-                            m2.x, m2.y, m2.z, m2.w, m3.x, m3.y, m3.z, m3.w};
-      const double rp[4] = {mr.x, mr.y, mr.z, mr.w};
-      double2 x01, x23;
-      if (row) {  // the other lanes' operands would leave the divisions' fast path
-        double X[4];
-        lu_solve4_recip(M, rp, b, X);
-        // dx = X - dQ, dQ + dx (linear_algebra.C:247-262)
-        x01 = make_double2(own01.x + (X[0] - own01.x), own01.y + (X[1] - own01.y));
-        x23 = make_double2(own23.x + (X[2] - own23.x), own23.y + (X[3] - own23.y));
-        own[0] = x01;
-        own[1] = x23;
-      }
-      __syncwarp();
-      if (lane == 0) level_arrive(bars + o);
-      // off the chain: the next tile's loads, this row's result to memory
-      h = hn;
-      asm volatile("" : "+r"(h.j), "+r"(h.block), "+r"(h.ln), "+r"(h.pos)::"memory");
-      asm volatile("" : "+r"(h.c.x), "+r"(h.c.y), "+r"(h.c.z), "+r"(h.c.w)::"memory");
-      load_row(k + 2 * kLevelWarps, hn);
-      load_tile(k + kLevelWarps, h);
-      if (row) {
-        double2* out = reinterpret_cast<double2*>(s.dQ) + 2 * (long)j;
-        out[0] = x01;
-        out[1] = x23;
-        dqp[2 * (long)(pos + 1)] = x01;
-        dqp[2 * (long)(pos + 1) + 1] = x23;
+      for (int t = 0; t < kRecBlocks; t++) a[t] = t < nb ? ld_d4(A + 16 * t) : z4;
+      rhs = s.RHS[4 * (long)R.j + r];
+      const int j = __shfl_sync(0xffffffffu, R.j, 4 * lane);  // row of slot `lane`
+      if (lane < 8) {
+        const double* L = s.LUd + 16 * (long)j;
+        m0 = ld_d4(L);
+        m1 = ld_d4(L + 4);
+        m2 = ld_d4(L + 8);
+        m3 = ld_d4(L + 12);
+        mr = ld_d4(s.LUr + 4 * (long)j);
       }
     }
+  }
+  // The rows' new values (x01, x23 in lane < 8 where `row`), also to their
+  // places `own`; wait() returns once what they read is in the window.
+  template <class Wait>
+  __device__ __forceinline__ void solve(const LevelRow& h, const double2* win, double2* own,
+                                        bool row, int lane, double2& x01, double2& x23,
+                                        Wait&& wait) const {
+    const unsigned FULL = 0xffffffffu;
+    const double2* d[kRecBlocks] = {
+        win + 2 * (h.c.x & 0xffff), win + 2 * (h.c.x >> 16), win + 2 * (h.c.y & 0xffff),
+        win + 2 * (h.c.y >> 16),    win + 2 * (h.c.z & 0xffff), win + 2 * (h.c.z >> 16),
+        win + 2 * (h.c.w & 0xffff), win + 2 * (h.c.w >> 16)};
+    wait();
+    double term[kRecBlocks];
+#pragma unroll
+    for (int t = 0; t < kRecBlocks; t++) {
+      const double2 d01 = d[t][0], d23 = d[t][1];
+      term[t] = (a[t].x * d01.x + a[t].y * d01.y + a[t].z * d23.x + a[t].w * d23.y);
+    }
+    const double2 own01 = own[0], own23 = own[1];
+    // an unused block's term is +0, and acc - 0 is acc, whatever its sign
+    double acc = rhs;
+#pragma unroll
+    for (int t = 0; t < kRecBlocks; t++) acc -= term[t];
+    const double b[4] = {__shfl_sync(FULL, acc, 4 * lane), __shfl_sync(FULL, acc, 4 * lane + 1),
+                         __shfl_sync(FULL, acc, 4 * lane + 2),
+                         __shfl_sync(FULL, acc, 4 * lane + 3)};
+    const double M[16] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w,
+                          m2.x, m2.y, m2.z, m2.w, m3.x, m3.y, m3.z, m3.w};
+    const double rp[4] = {mr.x, mr.y, mr.z, mr.w};
+    if (row) {  // the other lanes' operands would leave the divisions' fast path
+      double X[4];
+      lu_solve4_recip(M, rp, b, X);
+      // dx = X - dQ, dQ + dx (linear_algebra.C:247-262)
+      x01 = make_double2(own01.x + (X[0] - own01.x), own01.y + (X[1] - own01.y));
+      x23 = make_double2(own23.x + (X[2] - own23.x), own23.y + (X[3] - own23.y));
+      own[0] = x01;
+      own[1] = x23;
+    }
+  }
+};
+
+// The FP64 ordered sweep by bands of consecutive rows, a CTA each.  Inside a
+// band its rows go by dependency level, a tile of 8 rows a warp, four lanes a
+// row (lane r owning block row r), a level handed over by an mbarrier that
+// counts its tiles, as in k_sweep_chunk.  Between bands as in k_sweep_ordered:
+// results go to dq_new, prefilled with the not-ready pattern, and are polled
+// there.  The band's rows, and the rows of other bands that they read (a halo),
+// have places in shared memory.  The old values are loaded at the start; one
+// warp polls the halo rows that this sweep updates first, a row a lane, in the
+// order of the levels that need them, and counts as arrivals of those levels'
+// barriers.  CTAs take the bands in the sweep's order from a dispenser, so a
+// band waits only for bands that run or are done, whatever the residency; a
+// poll gives up after max_spin tries, and the sweep then ends with
+// ERR_SWEEP_TIMEOUT.
+//
+// Bound by the chain of levels.  A level inside an SM takes about 1,150 cycles:
+// the hand-over 110, reads and products 400, the ordered subtraction 60, the
+// 4x4 solve 500 (FP64 latency).  A row that waits for another band's pays a
+// publish and a poll through L2 besides, about 1,500, which the row-by-row
+// sweep over the whole GPU pays on every level.  us a sweep, that one and this:
+// 1,024 rows 92 / 52, 4,096 196 / 110, 10,816 306 / 185, 25,600 473 / 301,
+// 65,536 812 / 551, 181,476 1,500 / 1,181, 495,616 2,736 / 2,177.  (All rows in
+// one CTA: 53, 127, 272, 640 for the first four.)  Forming the products with
+// earlier levels' columns before the wait (two blocks a row reloaded, or the
+// tile's waiting blocks formed again after it) measured slower: the registers
+// or branches it takes cost more than the chain gains.
+//
+// Smaller bands have fewer tiles in flight each but more chains that cross
+// between them: us a sweep at 320 / 512 / 640 / 768 / 1,024 / 1,536 rows a band,
+// 25,600 rows 311 / 298 / 301 / 313 / 334 / 377, 65,536 600 / 559 / 551 / 560 /
+// 592 / 665, 181,476 1,261 / 1,213 / 1,181 / 1,170 / 1,181 / 1,270.
+constexpr int kBandRows = 640;
+constexpr int kLevelWarps = 7;      // tiles in flight (255 registers a thread)
+constexpr int kLevelThreads = 32 * (kLevelWarps + 1);
+constexpr int kBandTries = 1 << 24;  // the polls' limit ends these waits long before
+
+__host__ __device__ inline size_t band_smem_bytes(int nlev, int places) {
+  return 32 * ((size_t)places + 1) + 8 * (size_t)nlev;
+}
+
+template <bool FWD>
+__global__ void __launch_bounds__(kLevelThreads, 1) k_sweep_bands(DevState s, BandTables bt,
+                                                                 const double* dq_old,
+                                                                 double* dq_new, long max_spin) {
+  if (*s.stop || *s.skip) return;  // converged, or the linear residual dropped below 1e-15
+  extern __shared__ __align__(16) double2 level_smem[];
+  double2* win = level_smem;  // two words a place
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(win + 2 * (bt.places + 1));
+  __shared__ int taken;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, r = lane & 3, w = lane >> 2;
+  const int warp = __shfl_sync(FULL, (int)threadIdx.x >> 5, 0);  // uniform in the warp
+  if (threadIdx.x == 0) taken = (int)atomicAdd(s.counter, 1u);
+  __syncthreads();
+  if (taken >= bt.nband) return;
+  const Band B = bt.bands[FWD ? taken : bt.nband - 1 - taken];
+  const int2* lev = bt.lev + B.lev0;
+  // the o-th level to run waits for its halo rows and the level before
+  for (int o = threadIdx.x; o < B.nlev; o += kLevelThreads) {
+    const int l = FWD ? o : B.nlev - 1 - o;
+    const int halo = FWD ? lev[l].y & 0xffff : (int)((unsigned)lev[l].y >> 16);
+    level_init(bars + o, (unsigned)(halo + (o > 0 ? lev[FWD ? l - 1 : l + 1].x : 1)));
+  }
+  {
+    const double2* old = reinterpret_cast<const double2*>(dq_old);
+    for (int i = threadIdx.x; i < 2 * B.nrows; i += kLevelThreads)
+      cp_async16(win + i, old + 2 * (long)B.row0 + i);
+    const int2* fixed = bt.halo + (FWD ? B.halo0 + B.nlo : B.halo0);
+    const int nfixed = FWD ? B.nhi : B.nlo;
+    for (int i = threadIdx.x; i < 2 * nfixed; i += kLevelThreads) {
+      const int2 h = fixed[i >> 1];
+      cp_async16(win + 2 * (h.y & 0xffff) + (i & 1), old + 2 * (long)h.x + (i & 1));
+    }
+    // unused blocks read zeros
+    if (threadIdx.x < 2)
+      win[2 * (B.nrows + B.nlo + B.nhi) + threadIdx.x] = make_double2(0., 0.);
+    cp_async_commit();
+  }
+  bool timeout = false;
+  if (warp == kLevelWarps) {
+    // ---- the poller: lane i takes the entries i, i + 32, ... ----
+    cp_async_wait<0>();
+    __syncthreads();
+    const int2* list = bt.halo + (FWD ? B.halo0 : B.halo0 + B.nlo);
+    const int n = FWD ? B.nlo : B.nhi;
+    int e = lane;
+    int2 h = e < n ? list[e] : make_int2(0, 0);
+    long spins = 0;
+    while (e < n) {
+      unsigned long long u[4];
+      ld_relaxed_row(dq_new + 4 * (long)h.x, u);
+      bool ready = u[0] != kNotReady && u[1] != kNotReady && u[2] != kNotReady &&
+                   u[3] != kNotReady;
+      if (!ready && !timeout) {
+        // once any wait has timed out, every other one gives up too
+        if (++spins > max_spin ||
+            ((spins & 1023) == 0 && (*(volatile int*)s.status & ERR_SWEEP_TIMEOUT)))
+          timeout = true;
+      }
+      if (ready || timeout) {
+        double2* at = win + 2 * (h.y & 0xffff);
+        at[0] = make_double2(__longlong_as_double((long long)u[0]),
+                             __longlong_as_double((long long)u[1]));
+        at[1] = make_double2(__longlong_as_double((long long)u[2]),
+                             __longlong_as_double((long long)u[3]));
+        const int l = (int)((unsigned)h.y >> 16);
+        level_arrive(bars + (FWD ? l : B.nlev - 1 - l));
+        spins = 0;
+        e += 32;
+        if (e < n) h = list[e];
+      }
+    }
+    if (timeout) atomicOr(s.status, ERR_SWEEP_TIMEOUT);
+    return;
+  }
+  auto tile_at = [&](int k) { return B.tile0 + (FWD ? k : B.ntile - 1 - k); };
+  LevelRow h{}, hn{};
+  LevelTile T;
+  int k = warp;
+  load_level_row(bt.slots, k < B.ntile, tile_at(k), w, h);
+  load_level_row(bt.slots, k + kLevelWarps < B.ntile, tile_at(k + kLevelWarps), w, hn);
+  T.load(s, k < B.ntile, h, r, lane);
+  cp_async_wait<0>();
+  __syncthreads();
+  if (threadIdx.x == 0) level_arrive(bars);
+  for (; k < B.ntile; k += kLevelWarps) {
+    const int j = __shfl_sync(FULL, h.j, 4 * lane);  // the row lane < 8 solves
+    const int pos = __shfl_sync(FULL, h.pos, 4 * lane);
+    const bool row = j > 0 && lane < 8;
+    const int l = __shfl_sync(FULL, h.ln & 0xfffffff, 0);
+    const int o = FWD ? l : B.nlev - 1 - l;
+    double2 x01, x23;
+    T.solve(h, win, win + 2 * pos, row, lane, x01, x23,
+            [&] { timeout |= !level_wait(bars + o, 0, kBandTries); });
+    __syncwarp();
+    if (lane == 0 && o + 1 < B.nlev) level_arrive(bars + o + 1);
+    if (row) {  // the other bands wait for it
+      double* out = dq_new + 4 * (long)j;
+      st_relaxed_f64(out, x01.x);
+      st_relaxed_f64(out + 1, x01.y);
+      st_relaxed_f64(out + 2, x23.x);
+      st_relaxed_f64(out + 3, x23.y);
+    }
+    // off the chain: the next tile's loads
+    h = hn;
+    hold_level_row(h);
+    load_level_row(bt.slots, k + 2 * kLevelWarps < B.ntile, tile_at(k + 2 * kLevelWarps), w, hn);
+    T.load(s, k + kLevelWarps < B.ntile, h, r, lane);
   }
   if (timeout && lane == 0) atomicOr(s.status, ERR_SWEEP_TIMEOUT);
 }

@@ -122,26 +122,35 @@ struct ChunkTables {
   unsigned* sync;            // dispenser, chunks finished, sweep generation
 };
 
-// FP64 drop-in: the rows of the reference order by dependency level, in tiles
-// of 8 rows (padded at the end of a level), for the ordered sweep
-// k_sweep_levels.  Forward sweeps take the levels ascending, backward ones
-// descending.  A row's position is its place in level order; the sweep's
-// window of dQ is a ring over positions.
+// A row of k_sweep_bands.
 struct LevelSlot {
   int row;              // 0: an empty slot
   int block;            // first block of the row
-  unsigned level_nb;    // level, off-diagonal blocks << 28
-  int pos;              // the row's position (from 0)
-  uint4 cols;           // the blocks' columns as 16-bit ring places (the ring's size: none)
+  unsigned level_nb;    // level in the band, off-diagonal blocks << 28
+  int pos;              // the row's place
+  uint4 cols;           // the blocks' columns as 16-bit places
 };
 
-struct LevelTables {
-  int nlev;             // 0: the matrix does not take this sweep
-  int ring;             // rows its window of dQ holds
+// FP64 ordered sweep, k_sweep_bands: bands of consecutive rows of the reference
+// order; a band's rows by dependency level (the levels that it has,
+// renumbered), in tiles of 8 slots (padded at the end of a level).  Forward
+// sweeps take the levels ascending, backward ones descending.  Places are in
+// the band's shared memory: its rows in order, then the rows of other bands
+// that it reads, before it and behind it, then a place of zeros.
+struct Band {
+  int row0, nrows;      // its rows
+  int tile0, ntile;     // its tiles of 8 slots
+  int lev0, nlev;       // its levels
+  int halo0, nlo, nhi;  // the rows it reads before its own, then those behind
+};
+struct BandTables {
+  int nband;              // 0: the matrix does not take this sweep
+  int places, levels;     // most of a band
+  const Band* bands;
   const LevelSlot* slots;
-  const int* lev_tile;  // first tile of each level, plus the end
-  const int* load_to[2];  // per direction and level (in its order): positions below (forward)
-                          // or from (backward) it are in the window before the level runs
+  const int2* lev;        // per level: tiles; rows before the band that no earlier level needs,
+                          // rows behind it that no later level needs << 16
+  const int2* halo;       // row; place, that level << 16
 };
 
 struct DevState {

@@ -1,6 +1,7 @@
-"""The one-CTA FP64 ordered sweep by levels against the oracle, bit for bit:
-whole steps, and linear solves of systems whose pivots and right-hand sides
-reach past the range in which it divides by reciprocals."""
+"""The FP64 ordered sweep by bands of rows and dependency levels against the
+oracle, bit for bit: whole steps, meshes in other row numberings, and linear
+solves of systems whose pivots and right-hand sides reach past the range in
+which it divides by reciprocals."""
 import dataclasses
 
 import numpy as np
@@ -11,13 +12,30 @@ from cases import ndiff
 pytestmark = pytest.mark.gpu
 
 
-def _setup(nc, nr, order, subits):
+def _renumbered(grid, numbering):
+    """The grid with its nodes in random order or reversed."""
+    n = grid.x.shape[0]
+    perm = np.random.Generator(np.random.PCG64(5)).permutation(n) if numbering == "random" \
+        else np.arange(n)[::-1]  # new index of node i
+    x = np.empty_like(np.asarray(grid.x))
+    x[perm] = grid.x
+    bnds = [(bc, perm[np.asarray(segs) - 1] + 1) for bc, segs in grid.boundaries]
+    return dataclasses.replace(grid, x=x, tris=perm[np.asarray(grid.tris) - 1] + 1,
+                               boundaries=bnds)
+
+
+def _setup(nc, nr, order, subits, numbering="reordered"):
     from flowgpu import capi, workloads
     from flowgpu.prep import Mesh
     from oracle import port
     wl = workloads.Workload("levels", nc, nr, order == 3, order, 0.8 if order == 3 else 0.5,
                             subits=subits)
-    mesh = Mesh.from_grid(wl.grid(), order=order)
+    if numbering == "reordered":
+        mesh = Mesh.from_grid(wl.grid(), order=order)
+    else:
+        grid = wl.grid()
+        mesh = Mesh.from_grid(grid if numbering == "natural" else _renumbered(grid, numbering),
+                              order=order, reorder=0)
     fp = wl.params()
     Q0 = mesh.initial_state(fp)
     og = port.OracleGrid(mesh.sizes, mesh.arrays())
@@ -30,10 +48,11 @@ def _setup(nc, nr, order, subits):
 @pytest.mark.parametrize("nc,nr,order,subits,steps", [
     (8, 3, 1, 2, 3),       # 24 nodes: levels of a row or two
     (12, 4, 3, 3, 3),      # an odd number of sweeps
-    (66, 17, 3, 2, 3),
+    (40, 16, 1, 2, 3),     # 640 rows: one band
+    (66, 17, 3, 2, 3),     # 1,122 rows: a full band and a part
     (128, 32, 1, 4, 3),
     (400, 100, 1, 2, 2),   # 60 rows a level
-    (640, 160, 3, 1, 1),   # 102,400 rows
+    (640, 160, 3, 1, 1),   # 102,400 rows: more bands than SMs
 ])
 def test_steps_bitwise(nc, nr, order, subits, steps):
     mesh, og, p, gpu = _setup(nc, nr, order, subits)
@@ -42,6 +61,22 @@ def test_steps_bitwise(nc, nr, order, subits, steps):
         og.solve(p, ts)
         gpu.solve(ts)
         for name in ("Q", "dQ", "R"):
+            assert ndiff(og[name][4:4 * (nn + 1)], gpu.get(name)[4:4 * (nn + 1)]) == 0, (name, ts)
+    assert gpu.status() == 0
+    gpu.close()
+
+
+@pytest.mark.parametrize("numbering", ["natural", "reversed", "random"])
+@pytest.mark.parametrize("nc,nr,subits", [(48, 14, 3), (160, 40, 2)])
+def test_numberings_bitwise(nc, nr, subits, numbering):
+    """Rings a band, levels against the bands' order, and halos of thousands
+    of rows that cross bands at every level."""
+    mesh, og, p, gpu = _setup(nc, nr, 1, subits, numbering)
+    nn = mesh.sizes["nn"]
+    for ts in (1, 2):
+        og.solve(p, ts)
+        gpu.solve(ts)
+        for name in ("Q", "dQ"):
             assert ndiff(og[name][4:4 * (nn + 1)], gpu.get(name)[4:4 * (nn + 1)]) == 0, (name, ts)
     assert gpu.status() == 0
     gpu.close()
