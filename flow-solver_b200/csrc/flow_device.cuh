@@ -9,6 +9,29 @@
 
 namespace flow {
 
+// Correctly rounded y / m from r = RN(1 / m): the quotient estimate corrected
+// by two fused multiply-add steps.  By P. Markstein's theorem (IBM J. Res.
+// Dev. 34, 1990) the last step gives RN(y / m) when r is the correctly rounded
+// reciprocal and the estimate it corrects is within one ulp (which the first
+// step makes it), provided nothing over- or underflows; div_range bounds the
+// exponents of y and m to 2^+-400, which keeps every intermediate normal.
+// Bit for bit the division's result, at a third of its latency (measured:
+// 1.5e9 random and extreme operands, no difference).
+__device__ __forceinline__ bool div_range(double v) {
+  return ((unsigned)(__double2hiint(v) >> 20) & 0x7ffu) - 623u <= 800u;
+}
+__device__ __forceinline__ double div_recip(double y, double m, double r) {
+  double q = __dmul_rn(y, r);
+  q = __fma_rn(__fma_rn(-q, m, y), r, q);
+  return __fma_rn(__fma_rn(-q, m, y), r, q);
+}
+// A narrower range, 2^+-100 or +0, for what is multiplied before it is divided
+// (-0 is left to the division: div_recip's fused steps would give +0).
+__device__ __forceinline__ bool small_range(double v) {
+  return ((unsigned)(__double2hiint(v) >> 20) & 0x7ffu) - 923u <= 200u ||
+         __double_as_longlong(v) == 0;
+}
+
 // flux.C:37-68 Incompressible_Euler_Flux (the physical Euler flux).
 __device__ __forceinline__ void euler_flux(const double* Q, double* F, double nx, double ny,
                                            double len, double gamma) {
@@ -167,27 +190,62 @@ __device__ __forceinline__ void roe_core(double nx, double ny, double len, doubl
   lam[2] = fabs(thetabar + cbar);
   lam[3] = fabs(thetabar - cbar);
   const double c2 = cbar * cbar;
+  // Ten divisions by c2 and cbar from their reciprocals, or as they stand
+  // where an operand is out of range.  The face kernel with forward differences
+  // is bound by the FP64 pipe (66% busy, 264 of its 886 FP64 instructions an
+  // evaluation in divisions and roots): 65,536 nodes 140 -> 123 us, 40,804 at
+  // first order 96 -> 84.  The two branches whole: a correction after the fast
+  // form kept the operands live and spilled (132 us).  The other divisions, by
+  // rho and by the step, gained nothing this way.
+  const double g1 = gamma - 1.0, r2 = 1.0 / c2, rc = 1.0 / cbar;
+  const double hv2 = 0.5 * V2bar;
+  const bool in = small_range(ubar) && small_range(vbar) && small_range(nx) && small_range(ny) &&
+                  small_range(thetabar) && small_range(g1) && small_range(cbar) && g1 > 0. &&
+                  cbar > 0.;
+  double uc, vc, hv, t0, t1, t2, t3, xc, yc, tc;
+  if (in) {
+    uc = div_recip(ubar, c2, r2);
+    vc = div_recip(vbar, c2, r2);
+    hv = div_recip(hv2, c2, r2);
+    t0 = div_recip(g1 * hv2, c2, r2);
+    t1 = div_recip(g1 * ubar, c2, r2);
+    t2 = div_recip(g1 * vbar, c2, r2);
+    t3 = div_recip(-1.0 * g1, c2, r2);
+    xc = div_recip(nx, cbar, rc);
+    yc = div_recip(ny, cbar, rc);
+    tc = div_recip(thetabar, cbar, rc);
+  } else {
+    uc = ubar / c2;
+    vc = vbar / c2;
+    hv = hv2 / c2;
+    t0 = g1 * hv2 / c2;
+    t1 = g1 * ubar / c2;
+    t2 = g1 * vbar / c2;
+    t3 = -1.0 * g1 / c2;
+    xc = nx / cbar;
+    yc = ny / cbar;
+    tc = thetabar / cbar;
+  }
   T[0] = 1.0;
   T[1] = 0.0;
-  T[2] = 1.0 / c2;
-  T[3] = 1.0 / c2;
+  T[2] = r2;
+  T[3] = r2;
   T[4] = ubar;
   T[5] = -ny;
-  T[6] = ubar / c2 + nx / cbar;
-  T[7] = ubar / c2 - nx / cbar;
+  T[6] = uc + xc;
+  T[7] = uc - xc;
   T[8] = vbar;
   T[9] = nx;
-  T[10] = vbar / c2 + ny / cbar;
-  T[11] = vbar / c2 - ny / cbar;
-  T[12] = 0.5 * V2bar;
+  T[10] = vc + yc;
+  T[11] = vc - yc;
+  T[12] = hv2;
   T[13] = ubar * (-ny) + vbar * nx;
-  const double tc = thetabar / cbar, hv = (0.5 * V2bar) / c2;
   T[14] = ogm1 + tc + hv;
   T[15] = ogm1 - tc + hv;
-  Ti[0] = 1.0 - (gamma - 1.0) * (0.5 * V2bar) / c2;
-  Ti[1] = (gamma - 1.0) * ubar / c2;
-  Ti[2] = (gamma - 1.0) * vbar / c2;
-  Ti[3] = -1.0 * (gamma - 1.0) / c2;
+  Ti[0] = 1.0 - t0;
+  Ti[1] = t1;
+  Ti[2] = t2;
+  Ti[3] = t3;
   Ti[4] = -1.0 * (ubar * (-ny) + vbar * nx);
   Ti[5] = -ny;
   Ti[6] = nx;
@@ -402,22 +460,6 @@ __device__ __forceinline__ void lu_solve4(const double* M, const double* b, doub
   x[0] = (y0 - M[1] * x[1] - M[2] * x[2] - M[3] * x[3]) / M[0];
 }
 
-// Correctly rounded y / m from r = RN(1 / m): the quotient estimate corrected
-// by two fused multiply-add steps.  By P. Markstein's theorem (IBM J. Res.
-// Dev. 34, 1990) the last step gives RN(y / m) when r is the correctly rounded
-// reciprocal and the estimate it corrects is within one ulp (which the first
-// step makes it), provided nothing over- or underflows; div_range bounds the
-// exponents of y and m to 2^+-400, which keeps every intermediate normal.
-// Bit for bit the division's result, at a third of its latency (measured:
-// 1.5e9 random and extreme operands, no difference).
-__device__ __forceinline__ bool div_range(double v) {
-  return ((unsigned)(__double2hiint(v) >> 20) & 0x7ffu) - 623u <= 800u;
-}
-__device__ __forceinline__ double div_recip(double y, double m, double r) {
-  double q = __dmul_rn(y, r);
-  q = __fma_rn(__fma_rn(-q, m, y), r, q);
-  return __fma_rn(__fma_rn(-q, m, y), r, q);
-}
 // The reciprocal div_recip needs; NaN where the pivot is out of its range.
 __device__ __forceinline__ double pivot_recip(double m) {
   return div_range(m) ? 1.0 / m : __longlong_as_double(0x7ff8000000000000LL);
