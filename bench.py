@@ -277,7 +277,7 @@ def run_flow(args):
     achieved = bytes_per_sweep / (sweep_ms * 1e-3) / 1e9
     share = ms / max(sum(v[1] for v in ktimes.values()), 1e-30)
     traffic = ncu_traffic_per_sweep(wl.name)
-    roofline = {"bound": "hbm", "kernel": "k_sweep_ordered", "achieved": round(achieved, 2),
+    roofline = {"bound": "hbm", "kernel": "k_sweep_bands", "achieved": round(achieved, 2),
                 "peak": peaks["hbm_gbs"], "peak_kind": peak_kind, "unit": "GB/s",
                 "frac": round(achieved / peaks["hbm_gbs"], 5), "traffic": traffic,
                 "algorithmic_bytes_per_launch": bytes_per_sweep,

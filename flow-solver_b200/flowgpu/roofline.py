@@ -58,7 +58,7 @@ def colour_sweep_bytes(mesh) -> int:
 
 
 def ordered_sweep_bytes(mesh) -> int:
-    """One FP64 ordered sweep (k_sweep_ordered): per block 128 B of LHS and
+    """One FP64 ordered sweep (k_sweep_bands): per block 128 B of LHS and
     4 B of column index, per row RHS, LU of the diagonal, dQ read and write
     (132 B per block + 96 B per row, the diagonal block counted as a block)."""
     z = _sizes(mesh)
