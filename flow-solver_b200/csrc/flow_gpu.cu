@@ -1029,7 +1029,7 @@ bool preload_kernels() {
         (const void*)k_sweep_ordered32<false>, (const void*)k_prepare_sweep32,
         (const void*)k_fill_sweep_slots, (const void*)k_prepare_sweep,
         (const void*)k_lin_residual,
-        (const void*)k_finish_step,
+        (const void*)k_finish_step, (const void*)k_selftest_level_wait,
         (const void*)k_body_forces,
         (const void*)k_body_forces_sum})
     ok = ok && cudaFuncGetAttributes(&fa, f) == cudaSuccess;
@@ -2368,20 +2368,31 @@ int flow_selftest_sweep_timeout(flow_ctx* c, long max_spin, int* status) {
   cudaSetDevice(c->device);
   static const unsigned kFirst = 1;  // the dispenser starts at row 2: row 1 never runs
   reset_run(c, 0.);
+  // each part must report the time-out; other error bits are passed on
+  int seen = FLOW_ERR_SWEEP_TIMEOUT, other = 0;
+  auto part = [&]() {
+    const int st = read_status(c);
+    seen &= st;
+    other |= st & ~FLOW_ERR_SWEEP_TIMEOUT;
+    cudaMemsetAsync(c->s.status, 0, sizeof(int), c->stream);
+  };
   cudaMemsetAsync(c->s.status, 0, sizeof(int), c->stream);
   cudaMemsetAsync(c->s.skip, 0, sizeof(int), c->stream);
+  k_selftest_level_wait<<<1, 64, 0, c->stream>>>(c->s.status, (int)std::min(max_spin, 64L));
+  int rc = launch_check(c);
+  part();
   double* dq_new = c->s.dQ2;
   k_prepare_sweep<<<grid_blocks(4 * (c->nn + 1), 256), 256, 0, c->stream>>>(
       c->s, c->s.dQ, dq_new, 4 * (c->nn + 1));
-  int rc = launch_check(c);
+  rc |= launch_check(c);
   cudaMemcpyAsync(c->s.counter, &kFirst, sizeof(unsigned), cudaMemcpyHostToDevice, c->stream);
   k_sweep_ordered<true><<<c->nsm * 4, 128, 0, c->stream>>>(c->m, c->s, c->s.dQ, dq_new, max_spin);
   rc |= launch_check(c);
+  part();
   if (rc) return rc;
-  *status = read_status(c);
+  *status = seen | other;
   // the sweep's output buffer is scratch (the buffers were not swapped); the
   // context goes on from its state with a clear status
-  cudaMemsetAsync(c->s.status, 0, sizeof(int), c->stream);
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) return FLOW_ERR_CUDA;
   return 0;
 }

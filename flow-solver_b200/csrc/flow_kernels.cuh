@@ -1976,10 +1976,12 @@ __device__ __forceinline__ void level_arrive(unsigned long long* bar) {
                    static_cast<uint32_t>(__cvta_generic_to_shared(bar)))
                : "memory");
 }
-// Wait for the barrier's phase of this parity, at most kLevelTries tries (a
-// try itself waits a while in hardware); 0 when they run out.  The loop is
-// written in PTX so that its branches are uniform: the caller's exchanges
-// between lanes then need no reconvergence of the warp.
+// Wait for the barrier's phase of this parity, at most `left` tries (a try
+// itself waits a while in hardware); the tries left, 0 when they ran out.
+// Called by whole warps, and the same answer in every lane: a try may answer
+// the lanes of a warp differently, so they vote (all of them saw the phase
+// complete: leave), and the branches on the vote are uniform.  The caller's
+// exchanges between lanes then need no reconvergence of the warp.
 constexpr int kLevelTries = 1 << 16;
 __device__ __forceinline__ int level_wait(unsigned long long* bar, unsigned parity,
                                           int left = kLevelTries) {
@@ -1987,6 +1989,7 @@ __device__ __forceinline__ int level_wait(unsigned long long* bar, unsigned pari
       "{\n\t.reg .pred p, q;\n\t"
       "LEVEL_TRY:\n\t"
       "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\t"
+      "vote.sync.all.pred p, p, 0xffffffff;\n\t"
       "@p bra.uni LEVEL_DONE;\n\t"
       "sub.s32 %0, %0, 1;\n\t"
       "setp.gt.s32 q, %0, 0;\n\t"
@@ -1996,6 +1999,37 @@ __device__ __forceinline__ int level_wait(unsigned long long* bar, unsigned pari
       : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(bar))), "r"(parity)
       : "memory");
   return left;
+}
+
+// Self-test of level_wait, two warps: a wait for a barrier on which nobody
+// arrives ends after `tries` tries with 0 in every lane, and waits for barriers
+// that the other warp completes one after another end with the same tries left
+// in every lane.  Reports ERR_SWEEP_TIMEOUT when all of it held.
+constexpr int kSelftestLevels = 32;
+__global__ void __launch_bounds__(64) k_selftest_level_wait(int* status, int tries) {
+  __shared__ unsigned long long bars[kSelftestLevels + 1];
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x <= kSelftestLevels) level_init(bars + threadIdx.x, 1u);
+  __syncthreads();
+  if (threadIdx.x >= 32) {
+    for (int i = 0; i < kSelftestLevels; i++) {
+      if (lane == 0) {
+        __nanosleep(100 * (i & 7));
+        level_arrive(bars + i);
+      }
+      __syncwarp();
+    }
+    return;
+  }
+  bool ok = true;
+  for (int i = 0; i < kSelftestLevels; i++) {
+    const int left = level_wait(bars + i, 0), left0 = __shfl_sync(FULL, left, 0);
+    ok = ok && left > 0 && left == left0;
+  }
+  const int none = level_wait(bars + kSelftestLevels, 0, tries);
+  ok = ok && none == 0;
+  if (__all_sync(FULL, ok) && lane == 0) atomicOr(status, ERR_SWEEP_TIMEOUT);
 }
 
 // A chunk's levels in shared memory: one mbarrier each that counts the
