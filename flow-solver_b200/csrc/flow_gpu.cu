@@ -751,12 +751,15 @@ int begin_flags(const flow_ctx* c, const flow_params* p, const StepArgs& a) {
 // the run's first step is recognised on the device.  cont: the step enqueued
 // just before was this run's last with advance set, so nQ = Q already and the
 // step index and CFL are this step's; advance: a step with cont follows.
+// A run may start at or below step 0, whose steps take the index after the
+// previous one's: its step 1 sets the index to 1 by itself.
 int enqueue_step(flow_ctx* c, const flow_params* p, int ts, int hist_slot, int first,
                  bool device_ts = false, bool cont = false, bool advance = false) {
   int rc = 0;
   int total = c->nn + c->ng;
   c->citer = ts;
   if (device_ts) first = -1;
+  else if (ts == 1) cont = false;
   StepArgs a = make_args(p, ts);
   a.zero_iterate = 1;
   const int clear = begin_flags(c, p, a);
