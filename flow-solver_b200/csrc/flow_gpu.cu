@@ -668,7 +668,7 @@ int launch_linear_solve(flow_ctx* c, const flow_params* p, bool final_rms, bool 
     cudaMemsetAsync(c->s.dQ, 0, sizeof(double) * 4 * (c->nn + 1), c->stream);
     cudaMemsetAsync(c->s.skip, 0, sizeof(int), c->stream);
   }
-  const long max_spin = 1L << 21;  // ~0.1-0.2 s per wait at most
+  const long max_spin = 1L << 21;  // a wait ends after 0.6-0.7 s (measured, either sweep)
   for (int it = 0; it < p->subits; it++) {
     {
       Timed t(c, 4);
@@ -2369,7 +2369,8 @@ int flow_selftest_sweep_timeout(flow_ctx* c, long max_spin, int* status) {
     return FLOW_ERR_ARG;
   }
   cudaSetDevice(c->device);
-  static const unsigned kFirst = 1;  // the dispenser starts at row 2: row 1 never runs
+  // the dispensers start at 1: the sweep's first row, or its first band, never runs
+  static const unsigned kFirst = 1;
   reset_run(c, 0.);
   // each part must report the time-out; other error bits are passed on
   int seen = FLOW_ERR_SWEEP_TIMEOUT, other = 0;
@@ -2385,16 +2386,33 @@ int flow_selftest_sweep_timeout(flow_ctx* c, long max_spin, int* status) {
   int rc = launch_check(c);
   part();
   double* dq_new = c->s.dQ2;
-  k_prepare_sweep<<<grid_blocks(4 * (c->nn + 1), 256), 256, 0, c->stream>>>(
-      c->s, c->s.dQ, dq_new, 4 * (c->nn + 1));
-  rc |= launch_check(c);
-  cudaMemcpyAsync(c->s.counter, &kFirst, sizeof(unsigned), cudaMemcpyHostToDevice, c->stream);
-  k_sweep_ordered<true><<<c->nsm * 4, 128, 0, c->stream>>>(c->m, c->s, c->s.dQ, dq_new, max_spin);
-  rc |= launch_check(c);
-  part();
+  const int nd = 4 * (c->nn + 1);
+  auto sweep = [&](auto&& launch) {
+    k_prepare_sweep<<<grid_blocks(nd, 256), 256, 0, c->stream>>>(c->s, c->s.dQ, dq_new, nd);
+    rc |= launch_check(c);
+    cudaMemcpyAsync(c->s.counter, &kFirst, sizeof(unsigned), cudaMemcpyHostToDevice, c->stream);
+    launch();
+    rc |= launch_check(c);
+    part();
+  };
+  sweep([&] {
+    k_sweep_ordered<true><<<c->nsm * 4, 128, 0, c->stream>>>(c->m, c->s, c->s.dQ, dq_new, max_spin);
+  });
+  const BandTables& bt = c->bands;
+  if (bt.nband > 1) {  // one band polls for nothing
+    const size_t sm = band_smem_bytes(bt.levels, bt.places);
+    sweep([&] {
+      k_sweep_bands<true><<<bt.nband, kLevelThreads, sm, c->stream>>>(c->s, bt, c->s.dQ, dq_new,
+                                                                     max_spin);
+    });
+    sweep([&] {
+      k_sweep_bands<false><<<bt.nband, kLevelThreads, sm, c->stream>>>(c->s, bt, c->s.dQ, dq_new,
+                                                                      max_spin);
+    });
+  }
   if (rc) return rc;
   *status = seen | other;
-  // the sweep's output buffer is scratch (the buffers were not swapped); the
+  // the sweeps' output buffer is scratch (the buffers were not swapped); the
   // context goes on from its state with a clear status
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) return FLOW_ERR_CUDA;
   return 0;

@@ -408,11 +408,13 @@ const char *flow_last_error(void);
 /* Self-test of the sweeps' bounded waits (no counterpart in the reference).
  * First the wait for a dependency level inside a CTA: for one that nothing
  * completes it must give up after its tries, and every lane of the waiting
- * warp must get the same answer.  Then one forward ordered sweep whose
- * dispenser skips row 1, so the rows that depend on row 1 poll for a value
- * nothing writes until their spin limit (max_spin polls, at most 2^21),
- * report FLOW_ERR_SWEEP_TIMEOUT, publish a value so that nothing waits on
- * them, and the kernel ends.  *status receives FLOW_ERR_SWEEP_TIMEOUT when
+ * warp must get the same answer.  Then one forward row-by-row sweep whose
+ * dispenser skips row 1 and, where the context's FP64 sweep runs by bands of
+ * rows and there are two or more, one such sweep in each direction whose
+ * dispenser skips the first band.  What depends on the rows that never run
+ * polls for a value nothing writes until its spin limit (max_spin polls, at
+ * most 2^21), reports FLOW_ERR_SWEEP_TIMEOUT, publishes a value so that
+ * nothing waits on it, and each kernel ends.  *status receives FLOW_ERR_SWEEP_TIMEOUT when
  * every wait reported it, and any other status bits left; the call then
  * clears them.  The solution state is untouched and the context stays
  * usable.  Call it between steps. */
