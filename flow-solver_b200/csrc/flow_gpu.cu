@@ -19,6 +19,7 @@
 #include <type_traits>
 #include <map>
 #include <mutex>
+#include <new>
 #include <shared_mutex>
 #include <string>
 #include <vector>
@@ -184,7 +185,8 @@ struct flow_ctx {
   // one-CTA ordered sweep: stage tables (null when the matrix bandwidth is too
   // large for its dQ window, then the multi-CTA sweep is used)
   SweepTables sweep_tb{};
-  BandTables bands{};    // FP64 sweep by bands (build_bands); nband 0: not used
+  BandTables bands{};    // FP64 sweep by bands (ensure_bands); nband 0: not used
+  bool bands_tried = false;
   bool sweep_cta_ok = false;
   double* d_hist = nullptr;  // 2 x hist_cap device history of (dq, r_rho)
   int hist_cap = 0;
@@ -1088,7 +1090,6 @@ bool ensure_kernel_attrs(int device) {
 // and halo fit in shared memory.  Otherwise, and where the tables find no room,
 // the context keeps the grid-wide sweep.
 void build_bands(flow_ctx* c) {
-  if (c->bands.nband > 0) return;
   const int nn = c->nn;
   const std::vector<int>& ia = c->h_ia;
   const std::vector<int>& ja = c->h_ja;
@@ -1195,9 +1196,16 @@ void build_bands(flow_ctx* c) {
   std::copy(levs.begin(), levs.end(), at);
   std::copy(halo.begin(), halo.end(), at + nl);
   std::copy(bands.begin(), bands.end(), reinterpret_cast<Band*>(at + nl + nh));
+  // no room: the grid-wide sweep.  In an arena the tables leave as much free
+  // as the context holds, for what it may yet carve (other precision forms,
+  // saved states).
+  if (flow_arena* arena = c->buf.arena) {
+    std::lock_guard<std::mutex> lock(arena->mu);
+    if (arena->size - arena->used < slots.size() * sizeof(LevelSlot) + c->buf.bytes) return;
+  }
   const bool was = c->buf.carve_failed;
   const LevelSlot* d = upload_vec(c, slots);
-  if (!d) {  // no room: the grid-wide sweep
+  if (!d) {
     c->buf.carve_failed = was;
     return;
   }
@@ -1207,6 +1215,21 @@ void build_bands(flow_ctx* c) {
   bt.bands = reinterpret_cast<const Band*>(bt.halo + nh);
   bt.nband = nband;
   c->bands = bt;
+}
+
+// The band tables, once, before the first FP64 solve of a context (and so
+// before a chunk of its steps is captured): a context that only runs the
+// precision form or single stages needs none.  ms to create it and for its first
+// FP64 step, with the tables made at creation and so: 40,800 nodes k=1 42.2 +
+// 1.1 / 36.8 + 6.0, 65,536 k=2 113 + 1.5 / 105 + 9.9.  A matrix that does not
+// suit them is not looked at again.
+void ensure_bands(flow_ctx* c) {
+  if (c->bands_tried || c->precision != 0 || c->sweep_mode != 0) return;
+  c->bands_tried = true;
+  try {
+    build_bands(c);
+  } catch (const std::bad_alloc&) {  // no host memory: the grid-wide sweep
+  }
 }
 
 // Mode 3 reads none of the mode 1 / 2 tables: only the FP32 iterate.
@@ -1878,9 +1901,6 @@ static flow_ctx* create_impl(flow_arena* arena, const flow_grid_view* g, const f
   if (!upload(c, s.xn_bedges, xnb.data(), xnb.size() * 8) ||
       !upload(c, c->xnb0, xnb.data(), xnb.size() * 8))
     return fail(c, FLOW_ERR_CUDA, "upload failed");
-  // an arena's contexts mostly run the precision form: they build the FP64
-  // sweep's tables when they are set to precision 0
-  if (!arena) build_bands(c);
   // the context's own stream only: a device-wide synchronisation here would
   // invalidate a graph capture another thread has open
   if (cudaStreamSynchronize(c->stream) != cudaSuccess)
@@ -1949,10 +1969,6 @@ int flow_set_precision(flow_ctx* c, int mode) {
     int rc = mode == 3 ? build_chunk_iterate(c) : build_mixed_tables(c, mode >= 2);
     if (!rc && mode == 3) rc = build_chunk_tables(c);
     if (rc) return rc;
-  } else if (c->bands.nband == 0) {
-    cudaStreamSynchronize(c->stream);
-    drop_graphs(c);
-    build_bands(c);
   }
   c->precision = mode;
   return 0;
@@ -2119,6 +2135,7 @@ int flow_solve(flow_ctx* c, const flow_params* p, int ts, double* dq_norm, doubl
   if (rc) return rc;
   cudaSetDevice(c->device);
   if ((rc = ensure_hist(c, 1))) return rc;
+  ensure_bands(c);
   cudaEventRecord(c->ev0, c->stream);
   reset_run(c, 0.);
   rc = enqueue_step(c, p, ts, 0, 1);
@@ -2144,6 +2161,7 @@ int flow_run(flow_ctx* c, const flow_params* p, int ts0, int nsteps, double* r_h
   if (rc) return rc;
   cudaSetDevice(c->device);
   if ((rc = ensure_hist(c, std::max(nsteps, 1)))) return rc;
+  ensure_bands(c);
   cudaEventRecord(c->ev0, c->stream);
   reset_run(c, 0.);
   for (int i = 0; i < nsteps && !rc; i++)
@@ -2168,6 +2186,7 @@ int flow_converge(flow_ctx* c, const flow_params* p, int ts0, int max_steps, dou
   cudaSetDevice(c->device);
   if (chunk < 1) chunk = 64;
   if ((rc = ensure_hist(c, 1))) return rc;
+  ensure_bands(c);
   reset_run(c, drop);
   cudaEventRecord(c->ev0, c->stream);
   int done = 0, stop = 0, issued = 0;
@@ -2229,6 +2248,7 @@ int flow_converge_batch(flow_ctx** ctxs, int n, const flow_params* p, int ts0, i
     if (rc) return rc;
     cudaSetDevice(c->device);
     if ((rc = ensure_hist(c, 1))) return rc;
+    ensure_bands(c);
     if (!c->h_flags) {
       DeviceWide gate(g_device_gate);
       if (cudaHostAlloc(&c->h_flags, 2 * sizeof(int), cudaHostAllocDefault) != cudaSuccess)
@@ -2350,6 +2370,7 @@ int flow_linear_solve(flow_ctx* c, const flow_params* p, double* rms) {
   int rc = check_params(c, p);
   if (rc) return rc;
   cudaSetDevice(c->device);
+  ensure_bands(c);
   reset_run(c, 0.);
   rc = launch_linear_solve(c, p, true, false);
   if (rc) return rc;
@@ -2369,6 +2390,7 @@ int flow_selftest_sweep_timeout(flow_ctx* c, long max_spin, int* status) {
     return FLOW_ERR_ARG;
   }
   cudaSetDevice(c->device);
+  ensure_bands(c);
   // the dispensers start at 1: the sweep's first row, or its first band, never runs
   static const unsigned kFirst = 1;
   reset_run(c, 0.);
@@ -2671,6 +2693,7 @@ int flow_autotune(flow_ctx* c, const flow_params* p, int ts, int steps, int* var
   if (steps < 1) steps = 4;
   if ((rc = flow_save_state(c))) return rc;
   if ((rc = ensure_hist(c, 1))) return rc;
+  ensure_bands(c);
   const int saved_timing = c->timing;
   long kc[8];
   double km[8];
@@ -3066,6 +3089,7 @@ int begin_run(flow_ctx* c, const flow_params* p, double drop) {
   if (rc) return rc;
   cudaSetDevice(c->device);
   if ((rc = ensure_hist(c, 1))) return rc;
+  ensure_bands(c);
   if (!c->h_run) {
     DeviceWide gate(g_device_gate);
     if (cudaHostAlloc(&c->h_run, 6 * sizeof(int), cudaHostAllocDefault) != cudaSuccess ||
@@ -3080,6 +3104,11 @@ int begin_run(flow_ctx* c, const flow_params* p, double drop) {
   reset_run(c, drop);
   if (cudaEventRecord(c->ev0, c->stream) != cudaSuccess) return FLOW_ERR_CUDA;
   return 0;
+}
+
+void prepare_solve(flow_ctx* c) {
+  cudaSetDevice(c->device);
+  ensure_bands(c);
 }
 
 int enqueue_steps(flow_ctx* c, const flow_params* p, int ts0, int K) {

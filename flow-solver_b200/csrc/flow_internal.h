@@ -18,6 +18,9 @@ namespace internal {
 // may capture at once); the library's device-wide calls hold it exclusive.
 std::shared_mutex& device_gate();
 
+// What the context's solves need and lay out once (the FP64 sweep's tables),
+// ahead of its first run.
+void prepare_solve(flow_ctx* c);
 // Start a run on the context's stream: clear the stop flag and step count,
 // set the target drop of ||R_rho|| and record the run's start event.
 int begin_run(flow_ctx* c, const flow_params* p, double drop);

@@ -281,6 +281,7 @@ int flow_server_stage(flow_server* sv, const flow_grid_view* g, const flow_param
       }
     }
   }
+  if (!rc) flow::internal::prepare_solve(c);
   if (rc) {
     // the precision tables carved from the arena may not fit (FLOW_ERR_BUDGET);
     // every other failure is returned as it is

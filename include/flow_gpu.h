@@ -304,7 +304,15 @@ int flow_set_sweep_mode(flow_ctx *ctx, int mode);
  * by one CTA in the reference's order inside the chunk: close to the
  * reference order's convergence with a few launches per sweep.  It needs at
  * most 8 off-diagonal blocks per row and a matrix bandwidth whose chunk
- * windows fit in shared memory; otherwise switching to it fails. */
+ * windows fit in shared memory; otherwise switching to it fails.
+ * Mode 0's sweeps run by bands of rows where every row has at most 8
+ * off-diagonal blocks, and row by row otherwise; the same bits.  The bands'
+ * tables (about 45 to 110 bytes a row, by the mesh's numbering) are laid out
+ * once, by the context's first FP64 solve or run; a context that makes none
+ * does not hold them.  They come from the context's arena where it has one,
+ * and only while they leave as much of it free as the context holds; where
+ * they find no room the sweeps run row by row.  Setting the mode that the
+ * context is in takes no memory. */
 int flow_set_precision(flow_ctx *ctx, int mode);
 /* The context's precision mode (0..3; -1 for a null context). */
 int flow_precision_of(flow_ctx *ctx);
@@ -475,7 +483,8 @@ long long flow_arena_largest_free(flow_arena *arena);
  * with FLOW_ERR_CUDA for a CUDA error (a failed copy, a device fault). */
 flow_ctx *flow_create_in(flow_arena *arena, const flow_grid_view *g, const flow_params *p,
                          int *status);
-/* Device bytes a context holds. */
+/* Device bytes a context holds (they grow with the tables of a precision form,
+ * of the first FP64 solve, and with saved states). */
 long long flow_ctx_device_bytes(flow_ctx *ctx);
 
 /* ---- Serving engine (no counterpart in the reference) ---------------------
