@@ -498,20 +498,29 @@ int launch_residuals(flow_ctx* c, const StepArgs& a, int jac) {
   }
   // the approximate Roe Jacobian only in the precision form
   const bool approx = jac && c->jac_mode != 0 && c->precision != 0;
+  // the boundary edges in the flux launch's first blocks; by themselves while
+  // kernel classes are timed apart (flow_set_timing)
+  const int nbb = grid_blocks(c->nbe, 128), bnd = c->timing ? 0 : 1;
   {
     Timed t(c, 1);
-    const int nbs = grid_blocks(c->ns, 128) + grid_blocks(c->nbe, 128);
+    const int nbs = grid_blocks(c->ns, 128) + (bnd ? nbb : 0);
     launch_flux_variant(c->var[1], [&](auto V) {
       if (a.recon == 1) {
-        if (approx) k_subedge_flux<1, true, V.value, 1><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, 1);
-        else if (jac) k_subedge_flux<1, true, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, 1);
-        else k_subedge_flux<1, false, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, 1);
+        if (approx) k_subedge_flux<1, true, V.value, 1><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, bnd);
+        else if (jac) k_subedge_flux<1, true, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, bnd);
+        else k_subedge_flux<1, false, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, bnd);
       } else {
-        if (approx) k_subedge_flux<0, true, V.value, 1><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, 1);
-        else if (jac) k_subedge_flux<0, true, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, 1);
-        else k_subedge_flux<0, false, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, 1);
+        if (approx) k_subedge_flux<0, true, V.value, 1><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, bnd);
+        else if (jac) k_subedge_flux<0, true, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, bnd);
+        else k_subedge_flux<0, false, V.value><<<nbs, 128, 0, c->stream>>>(c->m, c->s, a, bnd);
       }
     });
+    rc |= launch_check(c);
+  }
+  if (!bnd && nbb > 0) {
+    Timed t(c, 2);
+    if (jac) k_boundary<true><<<nbb, 128, 0, c->stream>>>(c->m, c->s, a);
+    else k_boundary<false><<<nbb, 128, 0, c->stream>>>(c->m, c->s, a);
     rc |= launch_check(c);
   }
   {

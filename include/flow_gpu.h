@@ -402,7 +402,9 @@ int flow_restore_state(flow_ctx *ctx);
  * (off by default).  flow_kernel_times fills, per kernel class
  * (0 node_prepare, 1 subedge_flux, 2 boundary, 3 assemble, 4 sweep,
  * 5 lin_residual, 6 other), the number of launches and total milliseconds
- * since timing was switched on. */
+ * since timing was switched on.  While it is on the boundary edges are
+ * launched by themselves (class 2); otherwise they run in the first blocks of
+ * the flux launch.  The same bits. */
 int flow_set_timing(flow_ctx *ctx, int on);
 int flow_kernel_times(flow_ctx *ctx, long *launches, double *ms, int nclasses);
 
