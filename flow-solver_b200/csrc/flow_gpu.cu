@@ -3030,8 +3030,8 @@ extern "C" int flow_linear_residual_noalloc(const int* ia, const int* ja, const 
   if (nn < 1 || nn > FLOW_NOALLOC_MAX_ROWS) {
     char msg[160];
     snprintf(msg, sizeof msg,
-             "flow_linear_residual_noalloc: nn = %d rows is outside 1..%d, the rows its static "
-             "scratch holds",
+             "flow_linear_residual_noalloc: nn = %d rows is outside 1..%d, the limit of the "
+             "interface (its static scratch is the same for any rows)",
              nn, FLOW_NOALLOC_MAX_ROWS);
     set_error(msg);
     return FLOW_ERR_ARG;

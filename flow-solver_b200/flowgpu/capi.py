@@ -224,7 +224,7 @@ def linear_residual_noalloc(ia: int, ja: int, lhs: int, rhs: int, x: int, nn: in
                             stream: int | None = None) -> float:
     """b - A x RMS of a BCSR system in caller-held device memory (device
     pointers as ints), through flow_linear_residual_noalloc: no device
-    allocation, static scratch of FLOW_NOALLOC_MAX_ROWS rows."""
+    allocation, a static scratch; at most FLOW_NOALLOC_MAX_ROWS rows."""
     L = load()
     r = C.c_double()
     _check(L.flow_linear_residual_noalloc(ia, ja, lhs, rhs, x, int(nn), int(nnz), stream,
