@@ -1154,7 +1154,7 @@ def main():
     ap.add_argument("--sweep-dataflow", action="store_true",
                     help="with --profile-steps: one launch per mode 3 sweep (dataflow chunks)")
     ap.add_argument("--sweep-rows", type=int, default=0,
-                    help="with --profile-steps: sub-level rows of the mode 3 sweep ring (64, 32, 16)")
+                    help="with --profile-steps: CTA shape of the mode 3 sweep (64, 32, 16 for 16, 8, 4 warps)")
     ap.add_argument("--jacobian", type=int, default=0,
                     help="with --profile-steps: precision-form face Jacobians (flow_set_jacobian)")
     ap.add_argument("--node-variant", type=int, default=-1,

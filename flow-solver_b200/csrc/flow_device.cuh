@@ -13,10 +13,11 @@ namespace flow {
 // by two fused multiply-add steps.  By P. Markstein's theorem (IBM J. Res.
 // Dev. 34, 1990) the last step gives RN(y / m) when r is the correctly rounded
 // reciprocal and the estimate it corrects is within one ulp (which the first
-// step makes it), provided nothing over- or underflows; div_range bounds the
-// exponents of y and m to 2^+-400, which keeps every intermediate normal.
-// Bit for bit the division's result, at a third of its latency (measured:
-// 1.5e9 random and extreme operands, no difference).
+// step makes it; whether one step alone would do was not looked at), provided
+// nothing over- or underflows; div_range bounds the exponents of y and m to
+// 2^+-400, which keeps every intermediate normal.  Bit for bit the division's
+// result, at a third of its latency (measured: 1.5e9 random and extreme
+// operands, no difference).
 __device__ __forceinline__ bool div_range(double v) {
   return ((unsigned)(__double2hiint(v) >> 20) & 0x7ffu) - 623u <= 800u;
 }
@@ -196,7 +197,7 @@ __device__ __forceinline__ void roe_core(double nx, double ny, double len, doubl
   // evaluation in divisions and roots): 65,536 nodes 140 -> 123 us, 40,804 at
   // first order 96 -> 84.  The two branches whole: a correction after the fast
   // form kept the operands live and spilled (132 us).  The other divisions, by
-  // rho and by the step, gained nothing this way.
+  // rho and by the step, gained nothing with the two corrected steps.
   const double g1 = gamma - 1.0, r2 = 1.0 / c2, rc = 1.0 / cbar;
   const double hv2 = 0.5 * V2bar;
   const bool in = small_range(ubar) && small_range(vbar) && small_range(nx) && small_range(ny) &&

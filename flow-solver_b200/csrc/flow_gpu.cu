@@ -197,7 +197,7 @@ struct flow_ctx {
   int sched_sweeps = 0, sched_until = 0;  // sweep schedule (flow_set_sweep_schedule)
   MixedTables mt{};
   bool mt_ordered = false;  // tables in reference row order (modes 2, 3) or colour order (mode 1)
-  ChunkTables ct{};          // mode 3 tables and sweep records
+  ChunkTables ct{};          // mode 3 tables and sweep tiles
   std::vector<int> h_col_ptr, h_chunk_start;
   int chunk_rows = 0, chunk_levels = 0;  // requested limits (0: defaults)
   bool ring_ok[kRingShapes] = {};  // CTA shapes of the chunk sweep this mesh may take
@@ -1264,9 +1264,9 @@ int build_chunk_iterate(flow_ctx* c) {
 // bandwidth, at most 2048) or the level limit (default 32; a row's level is
 // one more than that of its latest in-chunk neighbour upstream, and the
 // longest chain is the same in both directions).  Colours: each chunk takes
-// the smallest colour no earlier adjacent chunk holds.  Records: per
-// direction, chunk by chunk, sub-levels of at most kRecRows rows of one
-// level, rows ascending inside a sub-level.
+// the smallest colour no earlier adjacent chunk holds.  Tiles: chunk by chunk,
+// level by level, a level's rows ascending and dealt 8 or 16 to a tile
+// (tile_rows); one copy serves both directions.
 int build_chunks_with(flow_ctx* c, int bw, int cmax, int lmax);
 
 int build_chunk_tables(flow_ctx* c) {

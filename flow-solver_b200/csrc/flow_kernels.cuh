@@ -1532,8 +1532,8 @@ __device__ __forceinline__ void st_relaxed_f64(double* p, double v) {
   asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
 
-// The four values of a row as one relaxed access (each value is single-copy
-// atomic by itself, which is all the ready pattern needs).
+// The four values of a row, a relaxed access each: a value is ready by itself,
+// and a row when none of its values is the not-ready pattern.
 __device__ __forceinline__ void ld_relaxed_row(const double* p, unsigned long long* u) {
   for (int i = 0; i < 4; i++) u[i] = ld_relaxed_u64(p + i);
 }
@@ -2431,20 +2431,20 @@ struct LevelTile {
 // poll gives up after max_spin tries and takes zeros, and the sweep then ends
 // with ERR_SWEEP_TIMEOUT.
 //
-// Bound by the chain of levels.  A level inside an SM takes about 1,150 cycles:
-// the hand-over 110, reads and products 400, the ordered subtraction 60, the
+// Bound by the chain of levels.  A level inside an SM takes about 1,175 cycles:
+// the hand-over 135 (25 of them the lanes' vote in level_wait), reads and products 400, the ordered subtraction 60, the
 // 4x4 solve 500 (FP64 latency).  A row that waits for another band's pays a
 // publish and a poll through L2 besides, about 1,500, which the row-by-row
 // sweep over the whole GPU pays on every level.  us a sweep, that one and this:
-// 1,024 rows 92 / 52, 4,096 196 / 110, 10,816 306 / 185, 25,600 473 / 301,
-// 65,536 812 / 551, 181,476 1,500 / 1,181, 495,616 2,736 / 2,177.  (All rows in
+// 1,024 rows 92 / 52, 4,096 196 / 113, 10,816 306 / 194, 25,600 473 / 306,
+// 65,536 812 / 562, 181,476 1,500 / 1,197, 495,616 2,736 / 2,201.  (All rows in
 // one CTA: 53, 127, 272, 640 for the first four.)  Forming the products with
 // earlier levels' columns before the wait (two blocks a row reloaded, or the
 // tile's waiting blocks formed again after it) measured slower: the registers
 // or branches it takes cost more than the chain gains.
 //
 // Smaller bands have fewer tiles in flight each but more chains that cross
-// between them: us a sweep at 320 / 512 / 640 / 768 / 1,024 / 1,536 rows a band,
+// between them: us a sweep (without the vote) at 320 / 512 / 640 / 768 / 1,024 / 1,536 rows a band,
 // 25,600 rows 311 / 298 / 301 / 313 / 334 / 377, 65,536 600 / 559 / 551 / 560 /
 // 592 / 665, 181,476 1,261 / 1,213 / 1,181 / 1,170 / 1,181 / 1,270.
 constexpr int kBandRows = 640;
