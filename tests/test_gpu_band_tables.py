@@ -138,3 +138,47 @@ def test_first_solve_as_replayed_chunks():
         assert _uses_bands(s) and s.status() == 0
         s.close()
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("room", ["much", "tight"])
+def test_fp64_requests_through_the_server(room):
+    """FP64 requests admitted from host threads beside running ones take the
+    steps that they take alone, with the tables and where they find no room."""
+    import concurrent.futures as cf
+    from flowgpu import capi
+    cases = [_case(64, 16), _case(96, 24), _case(40, 10), _case(128, 32)]
+    alone, need = [], 0
+    for mesh, fp in cases:
+        s = capi.Solver.from_mesh(mesh, fp, device=0)
+        need += _bytes(s) + (1 << 16)
+        s.set_state(mesh.initial_state(fp))
+        steps, _, _ = s.converge(1, 96, 1e-10, chunk=16, check=False)
+        alone.append((steps, s.get("Q")))
+        s.close()
+    arena = capi.Arena((1 << 30) if room == "much" else need)
+    srv = capi.Server(arena, chunk=16, max_slots=8)
+
+    def admit(i):
+        mesh, fp = cases[i]
+        while True:
+            slot = srv.submit(mesh, fp, mesh.initial_state(fp), precision=0, drop=1e-10,
+                              max_steps=96, tag=i)
+            if slot is not None:
+                return slot
+
+    got = {}
+    with cf.ThreadPoolExecutor(max_workers=4) as ex:
+        futs = [ex.submit(admit, i) for i in range(len(cases))]
+        while len(got) < len(cases):
+            for c in srv.progress(wait_us=500):
+                q, _ = srv.result(c["slot"])
+                srv.release(c["slot"])
+                got[c["tag"]] = (c["steps"], q)
+            for f in futs:
+                if f.done():
+                    f.result()
+    for i, (steps, q) in enumerate(alone):
+        assert got[i][0] == steps
+        assert np.array_equal(q[4:], got[i][1][4:])
+    srv.close()
+    arena.close()
